@@ -44,7 +44,32 @@ constexpr int NYS3 = (TY + 2) * TX;               // cells reconstructed in y
 constexpr int XF = TX + 1, NXF3 = TY * XF;        // x faces
 constexpr int NXFP3 = (NXF3 + 31) / 32 * 32;      // x faces padded to whole warps
 constexpr int NYF3 = (TY + 1) * TX;               // y faces
-constexpr int ZCHUNK = 64;  // z planes marched by one CTA
+constexpr int ZCHUNK = 64;  // most z planes marched by one CTA
+
+// z planes per CTA for a grid of `columns` columns and nz interior planes on a
+// device that runs `slots` CTAs at a time.  Every CTA costs its planes plus a
+// prologue (four plane loads and one z face, about kProloguePlanes planes), and
+// the launch as many rounds of CTAs as it takes, so the split with the smallest
+// rounds x (planes + prologue) is taken: small grids are cut into short chunks
+// until every SM has a CTA, large ones so that the last round is nearly full.
+// Against fixed chunks of 64 planes (ms per step on GB300): Harris 64x32x64 FP64
+// 12.3 -> 0.95 (8 CTAs before), field loop 100x100x200 FP64 15.9 -> 10.4 (208 CTAs
+// in two rounds), Harris 256x128x256 mixed 10.5 -> 9.4 (512 CTAs on 304 slots).
+constexpr double kProloguePlanes = 1.5;
+inline int pick_zchunk(long long columns, int nz, int slots) {
+  int best = ZCHUNK;
+  double best_cost = 1e300;
+  for (int c = nz < ZCHUNK ? nz : ZCHUNK; c >= 1; --c) {
+    const long long chunks = (nz + c - 1) / c;
+    if (chunks > 65535) break;  // gridDim.z
+    const double cost = (double)((columns * chunks + slots - 1) / slots) * (c + kProloguePlanes);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = c;
+    }
+  }
+  return best;
+}
 
 // ring of NRING primitive planes, then the x and y face states of one plane;
 // each face's flux overwrites the lower-cell face state that only it reads
@@ -163,7 +188,8 @@ __device__ __forceinline__ void load_plane(const StageArgs& a, T* W, int slot, i
 // shared memory each), so that one CTA's FP64 loads, updates and barriers
 // overlap the other's face work.
 template <class T, int FLUX>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 1) k_stage3d(const StageArgs a) {
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 1)
+    k_stage3d(const StageArgs a, const int zchunk) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* W = reinterpret_cast<T*>(smem_raw);  // [NRING][NV][PL]
   T* SLx = W + NRING * NV * PL;  // [NV][NXS3]; x fluxes in place
@@ -183,8 +209,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
   const size_t N = (size_t)ix * jx * kx;
   const int tid = threadIdx.x;
   const int gi0 = 1 + blockIdx.x * TX, gj0 = 1 + blockIdx.y * TY;
-  const int k0 = 1 + blockIdx.z * ZCHUNK;
-  const int k1 = min(k0 + ZCHUNK - 1, kx - 2);
+  const int k0 = 1 + blockIdx.z * zchunk;
+  const int k1 = min(k0 + zchunk - 1, kx - 2);
   const bool perx = a.bc_kind[0] == OMHD_BC_PERIODIC, pery = a.bc_kind[2] == OMHD_BC_PERIODIC;
   const bool perz = a.bc_kind[4] == OMHD_BC_PERIODIC;
   const bool resist = a.eta_kind != OMHD_ETA_NONE;
@@ -224,222 +250,232 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
   const double inv_dx = 1.0 / a.dx;
   const T inv_dx_t = T(inv_dx);
   if (sep_eta) {
-    for (int q = tid; q < 2 * (TX + 2) + 2 * (ZCHUNK + 2); q += NT) {
+    const int nez = k1 - k0 + 3;  // planes k0-1 .. k1+1
+    for (int q = tid; q < 2 * (TX + 2) + 2 * nez; q += NT) {
       if (q < 2 * (TX + 2)) {
         const int p = q % (TX + 2);
         const double x = a.xc[min(gi0 - 1 + p, ix - 1)] + (q >= TX + 2 ? 0.5 * a.dx : 0.0);
         (q < TX + 2 ? ex_c : ex_f)[p] = to_face<T>(exp(-(x * x) / 4.0));
       } else {
-        const int r = q - 2 * (TX + 2), p = r % (ZCHUNK + 2);
-        const double z = a.zc[min(k0 - 1 + p, kx - 1)] + (r >= ZCHUNK + 2 ? 0.5 * a.dx : 0.0);
-        (r < ZCHUNK + 2 ? ez_c : ez_f)[p] = to_face<T>(exp(-(z * z) / 4.0));
+        const int r = q - 2 * (TX + 2), p = r < nez ? r : r - nez;
+        const double z = a.zc[min(k0 - 1 + p, kx - 1)] + (r >= nez ? 0.5 * a.dx : 0.0);
+        (r < nez ? ez_c : ez_f)[p] = to_face<T>(exp(-(z * z) / 4.0));
       }
     }
   }
 
-  // ---- prologue: planes k0-2 .. k0+1, z face k0-1/2, cached upper state of cell k0 ----
+  // ---- prologue: planes k0-2 .. k0+1, then the z face k0-1/2 ----
   for (int p = k0 - 2; p <= k0 + 1; ++p)
     load_plane<T>(a, W, slot(p), p, gi0, gj0, perx, pery, perz, resist, glmf, p == k0);
   __syncthreads();
   T sLc[NV];  // z-upper face state of the current cell (k)
-  double Fzp[NV];  // z flux through face k-1/2
-  {
-    T L[NV], R[NV], Fo[NV];
+  double Fzp[NV] = {};  // z flux through face k-1/2
+  // The face below the chunk's first plane is solved by the loop's own code in a
+  // leading iteration k0-1 that does nothing else, so that a run's results do not
+  // depend on where the chunks begin.
+  const bool lead_in = sizeof(T) == 8 || (k0 - 1) % ZCHUNK != 0;
+  if (lead_in) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      T l, r;
-      reconstruct_t<T, OMHD_FAST>(lm, Wv(k0 - 2, v, oc), Wv(k0 - 1, v, oc), Wv(k0, v, oc), l, r);
-      L[v] = l;  // upper state of cell k0-1
-      reconstruct_t<T, OMHD_FAST>(lm, Wv(k0 - 1, v, oc), Wv(k0, v, oc), Wv(k0 + 1, v, oc), l, r);
-      R[v] = r;  // lower state of cell k0
-      sLc[v] = l;
-    }
-    if (!perz && k0 == 1) {  // bottom wall: VL = flip(VR)  (3D_reconnection_gpu/bc.cuf bc_for_H pattern)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) L[v] = ((a.bc_flip[4] >> v) & 1) ? -R[v] : R[v];
-    }
-    riemann_flux<T, 3, FLUX, OMHD_FAST>(L, R, ch, gam, r1, r2, Fo);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) Fzp[v] = to_f64<T>(Fo[v]);
-    if (resist && own) {  // z face k0-1/2 (flux_resistive.cuf:121-135)
-      const int k = k0 - 1;
-      if constexpr (sizeof(T) == 4) {
-        auto b = [&](int var, int dxo, int dyo, int dzo) { return Wv(k + dzo, var, oc + dxo + dyo * RX); };
-        const float eta_dx = sep_eta ? harris_eta_dx<T>(ex_c[tx + 1], ez_f[0], inv_dx_t)
-                                     : narrow_f64(eta3(a.eta_kind, a.xc[gi], a.yc[gj], a.zc[k] + 0.5 * a.dx) / a.dx);
-        resist_face_f32<3>(b, eta_dx, Fo);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) Fzp[v] = to_f64<T>(Fo[v]);
-      } else {
-        auto B = [&](int var, int dxo, int dyo, int dzo) { return to_f64<T>(Wv(k + dzo, var, oc + dxo + dyo * RX)); };
-        const double eta_dx = sep_eta ? harris_eta_dx<double>(ex_c[tx + 1], ez_f[0], inv_dx)
-                                      : eta3(a.eta_kind, a.xc[gi], a.yc[gj], a.zc[k] + 0.5 * a.dx) / a.dx;
-        const double JyS = (B(BX, 0, 0, 1) - B(BX, 0, 0, 0)) -
-                           0.25 * (B(BZ, 1, 0, 0) + B(BZ, 1, 0, 1) - B(BZ, -1, 0, 0) - B(BZ, -1, 0, 1));
-        const double JxS = -(B(BY, 0, 0, 1) - B(BY, 0, 0, 0)) +
-                           0.25 * (B(BZ, 0, 1, 0) + B(BZ, 0, 1, 1) - B(BZ, 0, -1, 0) - B(BZ, 0, -1, 1));
-        Fzp[EN] = Fzp[EN] + 0.5 * eta_dx * (JxS * (B(BY, 0, 0, 0) + B(BY, 0, 0, 1)) - JyS * (B(BX, 0, 0, 0) + B(BX, 0, 0, 1)));
-        Fzp[BX] = Fzp[BX] - eta_dx * JyS;
-        Fzp[BY] = Fzp[BY] + eta_dx * JxS;
-      }
+      T r;
+      reconstruct_t<T, OMHD_FAST>(lm, Wv(k0 - 2, v, oc), Wv(k0 - 1, v, oc), Wv(k0, v, oc), sLc[v], r);
     }
   }
   double vloc = 0.0;
 
-  for (int k = k0; k <= k1; ++k) {
+  for (int k = lead_in ? k0 - 1 : k0; k <= k1; ++k) {
+    const bool lead = k < k0;  // only the z face k+1/2 (uniform over the CTA)
     // Three CTA barriers per plane (plus one where a wall fix is needed).  The
     // ring slot of plane k+2 held plane k-2, whose last readers (the resistive
     // terms of plane k-1) finished before the previous plane's flux barrier;
     // the face arrays are rewritten only after the barrier that follows this
     // load, which every thread reaches after its reads of the previous plane's
-    // fluxes.  The prologue's z face reads plane k0-2: one barrier before the
-    // first load.
-    if (k == k0) __syncthreads();
-    load_plane<T>(a, W, slot(k + 2), k + 2, gi0, gj0, perx, pery, perz, resist, glmf, false);
-    __syncthreads();
-    if (k > k0) {
-      // positivity of the current plane's own cells (u2v.f90:36-45); plane k0
-      // was checked at load time in the prologue
-      if (own) {
-        const double ro = to_f64<T>(Wv(k, RO, oc)), pr = to_f64<T>(Wv(k, PR, oc));
-        if (pr <= 0)
-          raise_error(a.err, OMHD_NEG_PRESSURE, gi + 1, gj + 1, k + 1, 0, pr);
-        else if (ro <= 0)
-          raise_error(a.err, OMHD_NEG_DENSITY, gi + 1, gj + 1, k + 1, 0, ro);
-      }
-    }
-    const T* Wk = W + (size_t)slot(k) * NV * PL;
-
-    // ---- x and y face states of plane k, one phase ----
-    for (int q = tid; q < NXS3 + NYS3; q += NT) {
-      const bool xd = q < NXS3;
-      const int qq = xd ? q : q - NXS3;
-      int o, st;
-      if (xd) {  // x row cy, cells cx = 0..TX+1 (tile columns -1..TX)
-        const int cx = qq % XS, cy = qq / XS;
-        o = (cy + 2) * RX + (cx + 1);
-        st = 1;
-      } else {  // y column cx, cells cy = 0..TY+1 (tile rows -1..TY)
-        const int cx = qq % TX, cy = qq / TX;
-        o = (cy + 1) * RX + (cx + 2);
-        st = RX;
-      }
-      T* dl = xd ? SLx : SLy;
-      T* dr = xd ? SRx : SRy;
-      const int sv = xd ? NXS3 : NYS3;
+    // fluxes.  The chunk's first z face (and a seam's) reads plane k-2: one
+    // barrier before the load.
+    if (!lead) {
+      // FP32: the z face below every ZCHUNK-th plane enters that plane's update
+      // through this second copy of the solver, which the compiler contracts
+      // differently from the loop's; with chunks of ZCHUNK planes it was the first
+      // face of a chunk, and keeping it there gives a mixed run the same bits for
+      // every split
+      const bool seam = sizeof(T) == 4 && (k - 1) % ZCHUNK == 0;
+      if constexpr (sizeof(T) == 4) {
+        if (seam) {
+          T L[NV], R[NV], Fo[NV];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        T l, r;
-        reconstruct_t<T, OMHD_FAST>(lm, Wk[v * PL + o - st], Wk[v * PL + o], Wk[v * PL + o + st], l, r);
-        dl[v * sv + qq] = l;
-        dr[v * sv + qq] = r;
-      }
-    }
-    __syncthreads();
-    if (!perx || !pery) {  // wall face fixes, x by the first threads, y by the last
-      if (!perx && tid < TY * NV) {
-        const int cy = tid % TY, v = tid / TY;
-        if (gi0 == 1) {
-          const T s = SRx[v * NXS3 + cy * XS + 1];
-          SLx[v * NXS3 + cy * XS + 0] = ((a.bc_flip[0] >> v) & 1) ? -s : s;
+          for (int v = 0; v < NV; ++v) {
+            T l, r;
+            reconstruct_t<T, OMHD_FAST>(lm, Wv(k - 2, v, oc), Wv(k - 1, v, oc), Wv(k, v, oc), l, r);
+            L[v] = l;  // upper state of cell k-1
+            reconstruct_t<T, OMHD_FAST>(lm, Wv(k - 1, v, oc), Wv(k, v, oc), Wv(k + 1, v, oc), l, r);
+            R[v] = r;  // lower state of cell k
+            sLc[v] = l;
+          }
+          if (!perz && k == 1) {  // bottom wall: VL = flip(VR)  (3D_reconnection_gpu/bc.cuf bc_for_H pattern)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) L[v] = ((a.bc_flip[4] >> v) & 1) ? -R[v] : R[v];
+          }
+          riemann_flux<T, 3, FLUX, OMHD_FAST>(L, R, ch, gam, r1, r2, Fo);
+#pragma unroll
+          for (int v = 0; v < NV; ++v) Fzp[v] = to_f64<T>(Fo[v]);
+          if (resist && own) {  // z face k-1/2 (flux_resistive.cuf:121-135)
+            const int kl = k - 1;
+            auto b = [&](int var, int dxo, int dyo, int dzo) { return Wv(kl + dzo, var, oc + dxo + dyo * RX); };
+            const float eta_dx = sep_eta ? harris_eta_dx<T>(ex_c[tx + 1], ez_f[k - k0], inv_dx_t)
+                                         : narrow_f64(eta3(a.eta_kind, a.xc[gi], a.yc[gj], a.zc[kl] + 0.5 * a.dx) / a.dx);
+            resist_face_f32<3>(b, eta_dx, Fo);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) Fzp[v] = to_f64<T>(Fo[v]);
+          }
         }
-        const int cl = (ix - 2) - gi0 + 1;
-        if (cl >= 1 && cl <= TX) {
-          const T s = SLx[v * NXS3 + cy * XS + cl];
-          SRx[v * NXS3 + cy * XS + cl + 1] = ((a.bc_flip[1] >> v) & 1) ? -s : s;
+      }
+      if (k == k0 || seam) __syncthreads();
+      load_plane<T>(a, W, slot(k + 2), k + 2, gi0, gj0, perx, pery, perz, resist, glmf, false);
+      __syncthreads();
+      if (k > k0) {
+        // positivity of the current plane's own cells (u2v.f90:36-45); plane k0
+        // was checked at load time in the prologue
+        if (own) {
+          const double ro = to_f64<T>(Wv(k, RO, oc)), pr = to_f64<T>(Wv(k, PR, oc));
+          if (pr <= 0)
+            raise_error(a.err, OMHD_NEG_PRESSURE, gi + 1, gj + 1, k + 1, 0, pr);
+          else if (ro <= 0)
+            raise_error(a.err, OMHD_NEG_DENSITY, gi + 1, gj + 1, k + 1, 0, ro);
         }
       }
-      if (!pery && tid >= NT - TX) {
-        const int cx = tid - (NT - TX);
-        const int cl = (jx - 2) - gj0 + 1;
+      const T* Wk = W + (size_t)slot(k) * NV * PL;
+
+      // ---- x and y face states of plane k, one phase ----
+      for (int q = tid; q < NXS3 + NYS3; q += NT) {
+        const bool xd = q < NXS3;
+        const int qq = xd ? q : q - NXS3;
+        int o, st;
+        if (xd) {  // x row cy, cells cx = 0..TX+1 (tile columns -1..TX)
+          const int cx = qq % XS, cy = qq / XS;
+          o = (cy + 2) * RX + (cx + 1);
+          st = 1;
+        } else {  // y column cx, cells cy = 0..TY+1 (tile rows -1..TY)
+          const int cx = qq % TX, cy = qq / TX;
+          o = (cy + 1) * RX + (cx + 2);
+          st = RX;
+        }
+        T* dl = xd ? SLx : SLy;
+        T* dr = xd ? SRx : SRy;
+        const int sv = xd ? NXS3 : NYS3;
+  #pragma unroll
         for (int v = 0; v < NV; ++v) {
-          if (gj0 == 1) {
-            const T s = SRy[v * NYS3 + 1 * TX + cx];
-            SLy[v * NYS3 + 0 * TX + cx] = ((a.bc_flip[2] >> v) & 1) ? -s : s;
-          }
-          if (cl >= 1 && cl <= TY) {
-            const T s = SLy[v * NYS3 + cl * TX + cx];
-            SRy[v * NYS3 + (cl + 1) * TX + cx] = ((a.bc_flip[3] >> v) & 1) ? -s : s;
-          }
+          T l, r;
+          reconstruct_t<T, OMHD_FAST>(lm, Wk[v * PL + o - st], Wk[v * PL + o], Wk[v * PL + o + st], l, r);
+          dl[v * sv + qq] = l;
+          dr[v * sv + qq] = r;
         }
       }
       __syncthreads();
-    }
+      if (!perx || !pery) {  // wall face fixes, x by the first threads, y by the last
+        if (!perx && tid < TY * NV) {
+          const int cy = tid % TY, v = tid / TY;
+          if (gi0 == 1) {
+            const T s = SRx[v * NXS3 + cy * XS + 1];
+            SLx[v * NXS3 + cy * XS + 0] = ((a.bc_flip[0] >> v) & 1) ? -s : s;
+          }
+          const int cl = (ix - 2) - gi0 + 1;
+          if (cl >= 1 && cl <= TX) {
+            const T s = SLx[v * NXS3 + cy * XS + cl];
+            SRx[v * NXS3 + cy * XS + cl + 1] = ((a.bc_flip[1] >> v) & 1) ? -s : s;
+          }
+        }
+        if (!pery && tid >= NT - TX) {
+          const int cx = tid - (NT - TX);
+          const int cl = (jx - 2) - gj0 + 1;
+          for (int v = 0; v < NV; ++v) {
+            if (gj0 == 1) {
+              const T s = SRy[v * NYS3 + 1 * TX + cx];
+              SLy[v * NYS3 + 0 * TX + cx] = ((a.bc_flip[2] >> v) & 1) ? -s : s;
+            }
+            if (cl >= 1 && cl <= TY) {
+              const T s = SLy[v * NYS3 + cl * TX + cx];
+              SRy[v * NYS3 + (cl + 1) * TX + cx] = ((a.bc_flip[3] >> v) & 1) ? -s : s;
+            }
+          }
+        }
+        __syncthreads();
+      }
 
-    // ---- x and y fluxes of plane k, one phase (x faces padded to whole
-    // warps, so that no warp mixes directions); each flux replaces the
-    // lower-cell face state that only its own face reads ----
-    for (int q = tid; q < NXFP3 + NYF3; q += NT) {
-      if (q < NXFP3) {
-        if (q >= NXF3) continue;  // padding lanes
-        const int fx = q % XF, cy = q / XF;
-        T L[NV], R[NV], Fo[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          L[v] = SLx[v * NXS3 + cy * XS + fx];
-          R[v] = SRx[v * NXS3 + cy * XS + fx + 1];
-        }
-        riemann_flux<T, 1, FLUX, OMHD_FAST>(L, R, ch, gam, r1, r2, Fo);
-        if (resist) {  // flux_resistive.cuf:87-101
-          const int g = gi0 - 1 + fx, gjj = gj0 + cy;
-          if (g >= 0 && g <= ix - 2 && gjj <= jx - 2) {
-            const int o = (cy + 2) * RX + (fx + 1);
-            if constexpr (sizeof(T) == 4) {
-              auto b = [&](int var, int dxo, int dyo, int dzo) { return Wv(k + dzo, var, o + dxo + dyo * RX); };
-              const float eta_dx = sep_eta ? harris_eta_dx<T>(ex_f[fx], ez_c[k - k0 + 1], inv_dx_t)
-                                           : narrow_f64(eta3(a.eta_kind, a.xc[g] + 0.5 * a.dx, a.yc[gjj], a.zc[k]) / a.dx);
-              resist_face_f32<1>(b, eta_dx, Fo);
-            } else {
-              auto B = [&](int var, int dxo, int dyo, int dzo) { return to_f64<T>(Wv(k + dzo, var, o + dxo + dyo * RX)); };
-              const double eta_dx = sep_eta ? harris_eta_dx<double>(ex_f[fx], ez_c[k - k0 + 1], inv_dx)
-                                            : eta3(a.eta_kind, a.xc[g] + 0.5 * a.dx, a.yc[gjj], a.zc[k]) / a.dx;
-              const double JyS = -(B(BZ, 1, 0, 0) - B(BZ, 0, 0, 0)) +
-                                 0.25 * (B(BX, 0, 0, 1) + B(BX, 1, 0, 1) - B(BX, 0, 0, -1) - B(BX, 1, 0, -1));
-              const double JzS = (B(BY, 1, 0, 0) - B(BY, 0, 0, 0)) -
-                                 0.25 * (B(BX, 0, 1, 0) + B(BX, 1, 1, 0) - B(BX, 0, -1, 0) - B(BX, 1, -1, 0));
-              Fo[EN] = Fo[EN] + 0.5 * eta_dx * (JyS * (B(BZ, 0, 0, 0) + B(BZ, 1, 0, 0)) - JzS * (B(BY, 0, 0, 0) + B(BY, 1, 0, 0)));
-              Fo[BY] = Fo[BY] - eta_dx * JzS;
-              Fo[BZ] = Fo[BZ] + eta_dx * JyS;
+      // ---- x and y fluxes of plane k, one phase (x faces padded to whole
+      // warps, so that no warp mixes directions); each flux replaces the
+      // lower-cell face state that only its own face reads ----
+      for (int q = tid; q < NXFP3 + NYF3; q += NT) {
+        if (q < NXFP3) {
+          if (q >= NXF3) continue;  // padding lanes
+          const int fx = q % XF, cy = q / XF;
+          T L[NV], R[NV], Fo[NV];
+  #pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            L[v] = SLx[v * NXS3 + cy * XS + fx];
+            R[v] = SRx[v * NXS3 + cy * XS + fx + 1];
+          }
+          riemann_flux<T, 1, FLUX, OMHD_FAST>(L, R, ch, gam, r1, r2, Fo);
+          if (resist) {  // flux_resistive.cuf:87-101
+            const int g = gi0 - 1 + fx, gjj = gj0 + cy;
+            if (g >= 0 && g <= ix - 2 && gjj <= jx - 2) {
+              const int o = (cy + 2) * RX + (fx + 1);
+              if constexpr (sizeof(T) == 4) {
+                auto b = [&](int var, int dxo, int dyo, int dzo) { return Wv(k + dzo, var, o + dxo + dyo * RX); };
+                const float eta_dx = sep_eta ? harris_eta_dx<T>(ex_f[fx], ez_c[k - k0 + 1], inv_dx_t)
+                                             : narrow_f64(eta3(a.eta_kind, a.xc[g] + 0.5 * a.dx, a.yc[gjj], a.zc[k]) / a.dx);
+                resist_face_f32<1>(b, eta_dx, Fo);
+              } else {
+                auto B = [&](int var, int dxo, int dyo, int dzo) { return to_f64<T>(Wv(k + dzo, var, o + dxo + dyo * RX)); };
+                const double eta_dx = sep_eta ? harris_eta_dx<double>(ex_f[fx], ez_c[k - k0 + 1], inv_dx)
+                                              : eta3(a.eta_kind, a.xc[g] + 0.5 * a.dx, a.yc[gjj], a.zc[k]) / a.dx;
+                const double JyS = -(B(BZ, 1, 0, 0) - B(BZ, 0, 0, 0)) +
+                                   0.25 * (B(BX, 0, 0, 1) + B(BX, 1, 0, 1) - B(BX, 0, 0, -1) - B(BX, 1, 0, -1));
+                const double JzS = (B(BY, 1, 0, 0) - B(BY, 0, 0, 0)) -
+                                   0.25 * (B(BX, 0, 1, 0) + B(BX, 1, 1, 0) - B(BX, 0, -1, 0) - B(BX, 1, -1, 0));
+                Fo[EN] = Fo[EN] + 0.5 * eta_dx * (JyS * (B(BZ, 0, 0, 0) + B(BZ, 1, 0, 0)) - JzS * (B(BY, 0, 0, 0) + B(BY, 1, 0, 0)));
+                Fo[BY] = Fo[BY] - eta_dx * JzS;
+                Fo[BZ] = Fo[BZ] + eta_dx * JyS;
+              }
             }
           }
-        }
-#pragma unroll
-        for (int v = 0; v < NV; ++v) SLx[v * NXS3 + cy * XS + fx] = Fo[v];
-      } else {
-        const int qq = q - NXFP3;
-        const int cx = qq % TX, fy = qq / TX;
-        T L[NV], R[NV], Fo[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          L[v] = SLy[v * NYS3 + fy * TX + cx];
-          R[v] = SRy[v * NYS3 + (fy + 1) * TX + cx];
-        }
-        riemann_flux<T, 2, FLUX, OMHD_FAST>(L, R, ch, gam, r1, r2, Fo);
-        if (resist) {  // flux_resistive.cuf:104-118
-          const int gii = gi0 + cx, g = gj0 - 1 + fy;
-          if (g >= 0 && g <= jx - 2 && gii <= ix - 2) {
-            const int o = (fy + 1) * RX + (cx + 2);
-            if constexpr (sizeof(T) == 4) {
-              auto b = [&](int var, int dxo, int dyo, int dzo) { return Wv(k + dzo, var, o + dxo + dyo * RX); };
-              const float eta_dx = sep_eta ? harris_eta_dx<T>(ex_c[cx + 1], ez_c[k - k0 + 1], inv_dx_t)
-                                           : narrow_f64(eta3(a.eta_kind, a.xc[gii], a.yc[g] + 0.5 * a.dx, a.zc[k]) / a.dx);
-              resist_face_f32<2>(b, eta_dx, Fo);
-            } else {
-              auto B = [&](int var, int dxo, int dyo, int dzo) { return to_f64<T>(Wv(k + dzo, var, o + dxo + dyo * RX)); };
-              const double eta_dx = sep_eta ? harris_eta_dx<double>(ex_c[cx + 1], ez_c[k - k0 + 1], inv_dx)
-                                            : eta3(a.eta_kind, a.xc[gii], a.yc[g] + 0.5 * a.dx, a.zc[k]) / a.dx;
-              const double JxS = (B(BZ, 0, 1, 0) - B(BZ, 0, 0, 0)) -
-                                 0.25 * (B(BY, 0, 0, 1) + B(BY, 0, 1, 1) - B(BY, 0, 0, -1) - B(BY, 0, 1, -1));
-              const double JzS = -(B(BX, 0, 1, 0) - B(BX, 0, 0, 0)) +
-                                 0.25 * (B(BY, 1, 0, 0) + B(BY, 1, 1, 0) - B(BY, -1, 0, 0) - B(BY, -1, 1, 0));
-              Fo[EN] = Fo[EN] + 0.5 * eta_dx * (JzS * (B(BX, 0, 0, 0) + B(BX, 0, 1, 0)) - JxS * (B(BZ, 0, 0, 0) + B(BZ, 0, 1, 0)));
-              Fo[BX] = Fo[BX] + eta_dx * JzS;
-              Fo[BZ] = Fo[BZ] - eta_dx * JxS;
+  #pragma unroll
+          for (int v = 0; v < NV; ++v) SLx[v * NXS3 + cy * XS + fx] = Fo[v];
+        } else {
+          const int qq = q - NXFP3;
+          const int cx = qq % TX, fy = qq / TX;
+          T L[NV], R[NV], Fo[NV];
+  #pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            L[v] = SLy[v * NYS3 + fy * TX + cx];
+            R[v] = SRy[v * NYS3 + (fy + 1) * TX + cx];
+          }
+          riemann_flux<T, 2, FLUX, OMHD_FAST>(L, R, ch, gam, r1, r2, Fo);
+          if (resist) {  // flux_resistive.cuf:104-118
+            const int gii = gi0 + cx, g = gj0 - 1 + fy;
+            if (g >= 0 && g <= jx - 2 && gii <= ix - 2) {
+              const int o = (fy + 1) * RX + (cx + 2);
+              if constexpr (sizeof(T) == 4) {
+                auto b = [&](int var, int dxo, int dyo, int dzo) { return Wv(k + dzo, var, o + dxo + dyo * RX); };
+                const float eta_dx = sep_eta ? harris_eta_dx<T>(ex_c[cx + 1], ez_c[k - k0 + 1], inv_dx_t)
+                                             : narrow_f64(eta3(a.eta_kind, a.xc[gii], a.yc[g] + 0.5 * a.dx, a.zc[k]) / a.dx);
+                resist_face_f32<2>(b, eta_dx, Fo);
+              } else {
+                auto B = [&](int var, int dxo, int dyo, int dzo) { return to_f64<T>(Wv(k + dzo, var, o + dxo + dyo * RX)); };
+                const double eta_dx = sep_eta ? harris_eta_dx<double>(ex_c[cx + 1], ez_c[k - k0 + 1], inv_dx)
+                                              : eta3(a.eta_kind, a.xc[gii], a.yc[g] + 0.5 * a.dx, a.zc[k]) / a.dx;
+                const double JxS = (B(BZ, 0, 1, 0) - B(BZ, 0, 0, 0)) -
+                                   0.25 * (B(BY, 0, 0, 1) + B(BY, 0, 1, 1) - B(BY, 0, 0, -1) - B(BY, 0, 1, -1));
+                const double JzS = -(B(BX, 0, 1, 0) - B(BX, 0, 0, 0)) +
+                                   0.25 * (B(BY, 1, 0, 0) + B(BY, 1, 1, 0) - B(BY, -1, 0, 0) - B(BY, -1, 1, 0));
+                Fo[EN] = Fo[EN] + 0.5 * eta_dx * (JzS * (B(BX, 0, 0, 0) + B(BX, 0, 1, 0)) - JxS * (B(BZ, 0, 0, 0) + B(BZ, 0, 1, 0)));
+                Fo[BX] = Fo[BX] + eta_dx * JzS;
+                Fo[BZ] = Fo[BZ] - eta_dx * JxS;
+              }
             }
           }
+  #pragma unroll
+          for (int v = 0; v < NV; ++v) SLy[v * NYS3 + fy * TX + cx] = Fo[v];
         }
-#pragma unroll
-        for (int v = 0; v < NV; ++v) SLy[v * NYS3 + fy * TX + cx] = Fo[v];
       }
     }
     // ---- z face k+1/2 in registers: it reads only the ring, so the FP64 build
@@ -457,6 +493,12 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
         L[v] = sLc[v];
         R[v] = r;
         sLn[v] = l;
+      }
+      if constexpr (sizeof(T) == 8) {
+        if (!perz && k == 0) {  // bottom wall: VL = flip(VR)
+#pragma unroll
+          for (int v = 0; v < NV; ++v) L[v] = ((a.bc_flip[4] >> v) & 1) ? -R[v] : R[v];
+        }
       }
       if (!perz && k == kx - 2) {  // top wall: VR = flip(VL)
 #pragma unroll
@@ -489,18 +531,20 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
     };
     if constexpr (sizeof(T) == 8) z_face();
 
-    __syncthreads();
-    double acc[NV], gm[NV], gp[NV];
+    double acc[NV] = {}, gm[NV] = {}, gp[NV] = {};
+    if (!lead) {
+      __syncthreads();
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      acc[v] = to_f64<T>(SLx[v * NXS3 + ty * XS + tx]) - to_f64<T>(SLx[v * NXS3 + ty * XS + tx + 1]);
-      gm[v] = to_f64<T>(SLy[v * NYS3 + ty * TX + tx]);
-      gp[v] = to_f64<T>(SLy[v * NYS3 + (ty + 1) * TX + tx]);
+      for (int v = 0; v < NV; ++v) {
+        acc[v] = to_f64<T>(SLx[v * NXS3 + ty * XS + tx]) - to_f64<T>(SLx[v * NXS3 + ty * XS + tx + 1]);
+        gm[v] = to_f64<T>(SLy[v * NYS3 + ty * TX + tx]);
+        gp[v] = to_f64<T>(SLy[v * NYS3 + (ty + 1) * TX + tx]);
+      }
     }
     if constexpr (sizeof(T) == 4) z_face();
 
     // ---- update plane k ----
-    if (own) {
+    if (own && !lead) {
       const size_t c = (size_t)gi + (size_t)ix * ((size_t)gj + (size_t)jx * k);
       double out[NV];
 #pragma unroll
@@ -575,8 +619,14 @@ int launch_one3d(const StageArgs& a, cudaStream_t s) {
   static std::atomic<unsigned long long> configured{0};
   const int r = set_smem_attr_once(k_stage3d<T, FLUX>, bytes, configured);
   if (r) return r;
-  dim3 grid((a.ix - 2 + TX - 1) / TX, (a.jx - 2 + TY - 1) / TY, (a.kx - 2 + ZCHUNK - 1) / ZCHUNK);
-  k_stage3d<T, FLUX><<<grid, NT, bytes, s>>>(a);
+  int dev = 0, nsm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return (int)e;
+  dim3 grid((a.ix - 2 + TX - 1) / TX, (a.jx - 2 + TY - 1) / TY, 1);
+  const int zc = pick_zchunk((long long)grid.x * grid.y, a.kx - 2, nsm * (sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 1));
+  grid.z = (a.kx - 2 + zc - 1) / zc;
+  k_stage3d<T, FLUX><<<grid, NT, bytes, s>>>(a, zc);
   return (int)cudaGetLastError();
 }
 
