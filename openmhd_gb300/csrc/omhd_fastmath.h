@@ -1,45 +1,65 @@
-// omhd_fastmath.h -- FP64 reciprocal and reciprocal square root by
-// Newton-Raphson from hardware approximations, and binary32 <-> binary64
-// conversions on the integer pipe (device code).
+// omhd_fastmath.h -- FP64 reciprocal and square roots, and binary32 <-> binary64
+// conversions, on the integer pipes (device code).
 #pragma once
 
 namespace omhd {
 
 // ---------------------------------------------------------------------------
-// FP64 division and square root on a GPU whose FP64 pipe issues ~0.5 T
-// instructions/s: an IEEE divide costs ~4.4 FP64-pipe instruction slots and a
-// square root ~7 (measured on GB300).  The performance variants (FAST = true)
-// replace them by one higher-order refinement of a hardware approximation
-// from the special-function unit, which does not occupy the FP64 pipe:
-//   rcp_nr   : y0 = rcp.approx.ftz.f64(x) (relative error <= 2^-19.9,
-//              measured), e = 1 - x*y0 (one FMA, exact), then
-//              1/x = y0/(1-e) = y0*(1 + e + e^2 + O(e^3)): 3 FP64 operations,
-//              truncation ~e^3 ~ 2^-60 (the geometric series of 1/(1-e));
-//   rsqrt_nr : r0 = rsqrt.approx.ftz.f64(x) (relative error <= 2^-20.0,
-//              measured), e = 1 - x*r0^2, then
-//              1/sqrt(x) = r0*(1-e)^(-1/2) = r0*(1 + e/2 + 3e^2/8 + O(e^3)):
-//              5 FP64 operations, truncation ~(5/16)e^3 ~ 2^-62 (binomial
-//              series);
-//   sqrt_nr  : the same series applied to s0 = x*r0 ~ sqrt(x):
-//              sqrt(x) = s0*(1-e)^(-1/2) with e = 1 - s0*r0, 5 FP64
-//              operations.
-// Each returns a double within 1 ulp of the correctly rounded value (two
-// Newton-Raphson steps, the textbook alternative, cost 4 and 8 operations);
-// tests/test_gpu_fastmath.py enforces the 1-ulp bound on the GPU over
-// 2^-60..2^59 and over each function's whole domain.  The seeds flush
-// subnormal arguments, so rsqrt_nr and sqrt_nr take the IEEE operation outside
-// the positive normal range (a branch that the solver's positive normal
-// arguments never take); rcp_nr has no such branch and is meant for
-// |x| in [2^-1022, 2^1022] (x and 1/x normal); the solver's denominators
-// (densities, wave-speed differences, star-state factors) lie far inside it.  The parity variant (FAST = false) keeps the reference's
-// IEEE operations.
+// FP64 reciprocal and square roots without the FP64 pipe.  That pipe takes one
+// warp instruction in ~16 cycles (an SM issues 64 other ones in that time) and
+// bounds the FP64 kernels, so the performance variants (FAST = true) compute
+// 1/x, 1/sqrt(x) and sqrt(x) on the integer pipes: the argument's significand
+// as a 64-bit fixed-point number, a binary32 seed of the special-function unit
+// as a 32-bit one, and one third-order step of Newton's iteration (the series
+// of (1-e)^-1 and (1-e)^(-1/2) up to e^2) in 64-bit products:
+//   rcp_nr   : y0 <= 1/m from the seed, lowered by kSeedBias so that
+//              e = 1 - m*y0 is in [0, 2^-20); 1/m = y0*(1 + e + e^2 + O(e^3)),
+//              truncation below 2^-60;
+//   rsqrt_nr : e = 1 - m*y0^2 in [0, 2^-19), 1/sqrt(m) =
+//              y0*(1 + e/2 + 3e^2/8 + O(e^3)), truncation below 2^-58, with
+//              m in [1,4) and the exponent even;
+//   sqrt_nr  : m * 1/sqrt(m), the same series before it is rounded.
+// The 64-bit result is rounded once, to nearest: within 0.51 ulp (measured on
+// 6e7 arguments against extended precision; the FP64-pipe refinements these
+// replaced were within 1 ulp).  Measured on GB300 with 12 warps per SM, SM
+// cycles per warp operation: rcp 12.8, rsqrt 23, sqrt 27 (FP64-pipe forms: 52,
+// ~92, 92; a DFMA: 19), and beside a stream of DFMAs they cost no time at all
+// (16 DFMAs: 306 cycles; 16 DFMAs and 8 reciprocals: 305).
+// tests/test_gpu_fastmath.py enforces 1 ulp over 2^-60..2^59 and over each
+// function's whole domain: |x| in [2^-1022, 2^1022] for rcp_nr (x and 1/x
+// normal; zero, subnormal and larger arguments, infinities and NaN give NaN),
+// positive normal x for the square roots, which take the IEEE operation outside
+// it (a branch that the solver's arguments never take).  The parity variant
+// (FAST = false) keeps the reference's IEEE operations.
+//
+// rcp_nr_fp, rsqrt_nr_fp and sqrt_nr_fp are the refinements on the FP64 pipe (3,
+// 5 and 5 operations from a binary64 seed, within 1 ulp).  The FP32-mixed kernels keep them for the
+// CFL speed: another rounding of dt moves every cell of a mixed run by an ulp,
+// and a state that differs in its last bit now and then rounds to the
+// neighbouring binary32 number.
 // ---------------------------------------------------------------------------
 #ifdef __CUDACC__
+constexpr unsigned kSeedBias = 1100u;  // in units of 2^-32; seed error <= 2^-23 + 2^-23 relative (1024 units)
+
+// a seed r in [1/2, 1] (its binary32 bits) as a 0.32 fixed-point number, lowered by kSeedBias
+__device__ __forceinline__ unsigned seed_fixed(float r) {
+  return __float_as_uint(r) * 256u + (0x80000000u - kSeedBias);
+}
+
 __device__ __forceinline__ double rcp_nr(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(fma(e, e, e), y, y);
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned mh = __funnelshift_l(lo, hi, 11) | 0x80000000u, ml = lo << 11;  // m = mh:ml * 2^-63 in [1,2)
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float((mh >> 8) + 0x3f000000u)));
+  const unsigned y0 = seed_fixed(r);
+  const unsigned long long e = 0x8000000000000000ull - ((unsigned long long)mh * y0 + __umulhi(ml, y0));  // e * 2^63
+  const unsigned e32 = __funnelshift_r((unsigned)e, (unsigned)(e >> 32), 11);                             // e * 2^52
+  const unsigned long long s = e + 0x8000000000000000ull + (__umulhi(e32, e32) >> 9);  // (1 + e + e^2) * 2^63
+  const unsigned long long t = (unsigned long long)y0 * (unsigned)(s >> 32) + __umulhi(y0, (unsigned)s);  // y * 2^63
+  const unsigned long long q = (t + 512u) >> 10;  // 53 bits (2^53 where y rounds to 1)
+  const unsigned f = hi & 0xfff00000u;            // sign and exponent
+  const unsigned rh = (f & 0x7ff00000u) - 0x00100000u < 0x7fd00000u ? 0x7fc00000u - f + (unsigned)(q >> 32) : 0x7ff80000u;
+  return __hiloint2double((int)rh, (int)(unsigned)q);
 }
 
 // x positive, normal and finite (one integer compare on the bit pattern)
@@ -48,7 +68,55 @@ __device__ __forceinline__ bool pos_normal(double x) {
   return b - 0x0010000000000000ULL < 0x7fe0000000000000ULL;
 }
 
+// x = m 4^q with m = mh:ml * 2^-62 in [1,4); t = 2^63 / sqrt(m); the exponent
+// field of 2^q, less that of 1/2, as ex (positive normal x)
+__device__ __forceinline__ void rsqrt_fixed(double x, unsigned& mh, unsigned& ml, unsigned long long& t, unsigned& ex) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned sh = 11u - ((hi >> 20) & 1u);
+  mh = __funnelshift_l(lo, (hi & 0xfffffu) | 0x100000u, sh);
+  ml = lo << sh;
+  const unsigned g = (__funnelshift_l(lo, hi, 3) & 0xffffffu) ^ 0x800000u;  // significand and exponent parity
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(g + 0x3f800000u)));
+  const unsigned y0 = seed_fixed(r);
+  const unsigned long long y2 = (unsigned long long)y0 * y0;
+  const unsigned y2h = (unsigned)(y2 >> 32);
+  const unsigned long long e =
+      0x4000000000000000ull - ((unsigned long long)mh * y2h + __umulhi(mh, (unsigned)y2) + __umulhi(ml, y2h));  // e * 2^62
+  const unsigned e32 = __funnelshift_r((unsigned)e, (unsigned)(e >> 32), 11);                                   // e * 2^51
+  const unsigned long long s = e + 0x8000000000000000ull + __umulhi(__umulhi(e32, e32), 3u << 22);  // (1 + e/2 + 3e^2/8) * 2^63
+  t = (unsigned long long)y0 * (unsigned)(s >> 32) + __umulhi(y0, (unsigned)s);
+  ex = ((hi + 0x100000u) >> 1) & 0xfff00000u;
+}
+
 __device__ __forceinline__ double rsqrt_nr(double x) {
+  if (!pos_normal(x)) return 1.0 / sqrt(x);
+  unsigned mh, ml, ex;
+  unsigned long long t;
+  rsqrt_fixed(x, mh, ml, t, ex);
+  const unsigned long long q = (t + 512u) >> 10;
+  return __hiloint2double((int)((1533u << 20) - ex + (unsigned)(q >> 32)), (int)(unsigned)q);
+}
+
+__device__ __forceinline__ double sqrt_nr(double x) {
+  if (!pos_normal(x)) return sqrt(x);
+  unsigned mh, ml, ex;
+  unsigned long long t;
+  rsqrt_fixed(x, mh, ml, t, ex);
+  const unsigned th = (unsigned)(t >> 32);
+  const unsigned long long p = (unsigned long long)mh * th + __umulhi(mh, (unsigned)t) + __umulhi(ml, th);  // sqrt(m) * 2^61
+  const unsigned long long q = (p + 256u) >> 9;
+  return __hiloint2double((int)((510u << 20) + ex + (unsigned)(q >> 32)), (int)(unsigned)q);
+}
+
+__device__ __forceinline__ double rcp_nr_fp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(fma(e, e, e), y, y);
+}
+
+__device__ __forceinline__ double rsqrt_nr_fp(double x) {
   if (!pos_normal(x)) return 1.0 / sqrt(x);
   double r;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -56,7 +124,7 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
   return fma(r * e, fma(0.375, e, 0.5), r);
 }
 
-__device__ __forceinline__ double sqrt_nr(double x) {
+__device__ __forceinline__ double sqrt_nr_fp(double x) {
   if (!pos_normal(x)) return sqrt(x);
   double r;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));

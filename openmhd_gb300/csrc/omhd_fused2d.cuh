@@ -691,15 +691,15 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
 
     if (stage2) {  // set_dt.f90:27-37 on the new state
       const double ro = out[RO];
-      const double iro = rcp_<double, OMHD_FAST>(ro);  // one reciprocal for the three velocities
+      const double iro = rcp_<double, OMHD_FAST, sizeof(T) == 4>(ro);  // one reciprocal for the three velocities
       const double vx = divr_<double, OMHD_FAST>(out[MX], ro, iro), vy = divr_<double, OMHD_FAST>(out[MY], ro, iro),
                    vz = divr_<double, OMHD_FAST>(out[MZ], ro, iro);
       const double rv2 = vx * out[MX] + vy * out[MY] + vz * out[MZ];
       const double B2 = out[BX] * out[BX] + out[BY] * out[BY] + out[BZ] * out[BZ];
       const double pr = f1g * (out[EN] - 0.5 * (rv2 + B2));
       const double f1 = gamma * pr;
-      const double vfx = fast_speed<double, OMHD_FAST>(f1, B2, out[BX], ro);
-      const double vfy = fast_speed<double, OMHD_FAST>(f1, B2, out[BY], ro);
+      const double vfx = fast_speed<double, OMHD_FAST, sizeof(T) == 4>(f1, B2, out[BX], ro);
+      const double vfy = fast_speed<double, OMHD_FAST, sizeof(T) == 4>(f1, B2, out[BY], ro);
       const double sx = fabs(vx) + vfx, sy = fabs(vy) + vfy;
       const double sc = lt_<double, OMHD_FAST>(sx, sy) ? sy : sx;  // fmax2(sx, sy)
       vcell = lt_<double, OMHD_FAST>(vcell, sc) ? sc : vcell;

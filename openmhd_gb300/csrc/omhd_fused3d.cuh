@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
           }
       if (a.stage == 2) {  // 3D_basic/set_dt.f90:27-43 on the new state
         const double ro = out[RO];
-        const double iro = rcp_<double, OMHD_FAST>(ro);  // one reciprocal for the three velocities
+        const double iro = rcp_<double, OMHD_FAST, sizeof(T) == 4>(ro);  // one reciprocal for the three velocities
         const double vx = divr_<double, OMHD_FAST>(out[MX], ro, iro), vy = divr_<double, OMHD_FAST>(out[MY], ro, iro), vz = divr_<double, OMHD_FAST>(out[MZ], ro, iro);
         const double rv2 = vx * out[MX] + vy * out[MY] + vz * out[MZ];
         const double B2 = out[BX] * out[BX] + out[BY] * out[BY] + out[BZ] * out[BZ];
@@ -592,9 +592,9 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
         const double f1 = gamma * pr;
         // fmax2 of the three speeds and of the running max, the comparisons on
         // the integer pipe in the FAST builds (same results)
-        const double sx = fabs(vx) + fast_speed<double, OMHD_FAST>(f1, B2, out[BX], ro);
-        const double sy = fabs(vy) + fast_speed<double, OMHD_FAST>(f1, B2, out[BY], ro);
-        const double sz = fabs(vz) + fast_speed<double, OMHD_FAST>(f1, B2, out[BZ], ro);
+        const double sx = fabs(vx) + fast_speed<double, OMHD_FAST, sizeof(T) == 4>(f1, B2, out[BX], ro);
+        const double sy = fabs(vy) + fast_speed<double, OMHD_FAST, sizeof(T) == 4>(f1, B2, out[BY], ro);
+        const double sz = fabs(vz) + fast_speed<double, OMHD_FAST, sizeof(T) == 4>(f1, B2, out[BZ], ro);
         double s = lt_<double, OMHD_FAST>(sx, sy) ? sy : sx;
         s = lt_<double, OMHD_FAST>(s, sz) ? sz : s;
         vloc = lt_<double, OMHD_FAST>(s, vloc) ? vloc : s;

@@ -60,10 +60,11 @@ __device__ __forceinline__ bool lt_(T a, T b) {  // a < b
   return a < b;
 }
 
-// a / b and 1 / b under the variant's policy
-template <class T, bool FAST>
+// a / b and 1 / b under the variant's policy (FPIPE: the refinement on the FP64
+// pipe, which the FP32-mixed kernels keep for the CFL speed)
+template <class T, bool FAST, bool FPIPE = false>
 __device__ __forceinline__ T rcp_(T b) {
-  if constexpr (FAST && sizeof(T) == 8) return rcp_nr(b);
+  if constexpr (FAST && sizeof(T) == 8) return FPIPE ? rcp_nr_fp(b) : rcp_nr(b);
   return T(1) / b;
 }
 template <class T, bool FAST>
@@ -71,21 +72,20 @@ __device__ __forceinline__ T div_(T a, T b) {
   if constexpr (FAST && sizeof(T) == 8) return a * rcp_nr(b);
   return a / b;
 }
-// square root under the variant's policy: sqrt_nr for FAST FP64 (5 FP64-pipe
-// operations instead of ~7 for the IEEE sqrt; within ~1 ulp; IEEE outside the
+// square root under the variant's policy: sqrt_nr for FAST FP64 (IEEE outside the
 // positive normal range, so sqrt(+-0) = +-0)
-template <class T, bool FAST>
+template <class T, bool FAST, bool FPIPE = false>
 __device__ __forceinline__ T sqrt_(T x) {
-  if constexpr (FAST && sizeof(T) == 8) return sqrt_nr(x);
+  if constexpr (FAST && sizeof(T) == 8) return FPIPE ? sqrt_nr_fp(x) : sqrt_nr(x);
   return sqrt(x);
 }
 // sqrt(a / b) for a, b > 0: a * (1/sqrt(a*b)) for FAST FP64 (one product and
 // one rsqrt refinement replace a division and a square root), IEEE otherwise
-template <class T, bool FAST>
+template <class T, bool FAST, bool FPIPE = false>
 __device__ __forceinline__ T sqrt_ratio_(T a, T b) {
   if constexpr (FAST && sizeof(T) == 8) {
     const double ab = a * b;
-    return pos_normal(ab) ? a * rsqrt_nr(ab) : sqrt(a / b);
+    return pos_normal(ab) ? a * (FPIPE ? rsqrt_nr_fp(ab) : rsqrt_nr(ab)) : sqrt(a / b);
   }
   return sqrt(a / b);
 }
@@ -867,11 +867,11 @@ __device__ __forceinline__ void u2v_cell(const double (&u)[NV], double f1g, floa
 }
 
 // Fast magnetosonic speed used by set_dt (2D_basic/set_dt.f90:27-34).
-template <class T, bool FAST = false>
+template <class T, bool FAST = false, bool FPIPE = false>
 __device__ __forceinline__ T fast_speed(T f1, T B2, T bd, T ro) {
   const T f2 = 4 * f1 * (bd * bd);
   const T D = (f1 + B2) * (f1 + B2) - f2;
-  return sqrt_ratio_<T, FAST>((f1 + B2) + sqrt_<T, FAST>(lt0_<T, FAST>(D) ? T(0) : D), 2 * ro);
+  return sqrt_ratio_<T, FAST, FPIPE>((f1 + B2) + sqrt_<T, FAST, FPIPE>(lt0_<T, FAST>(D) ? T(0) : D), 2 * ro);
 }
 
 }  // namespace omhd
