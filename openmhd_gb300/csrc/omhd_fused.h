@@ -43,6 +43,7 @@ struct StageArgs {
   // 1/(gamma-1), gamma/(gamma-1) (flux_solver.f90:38-39) in FP64 and, with
   // gamma, rounded to binary32 for the FP32 face arithmetic
   double sdx, sdy, sdz;
+  double ryx, rzx;     // dx/dy, dx/dz: the weights of the y and z flux differences beside the x ones (1 on iso grids)
   double gm1, r1, r2;  // gamma - 1 (u2v.f90:11), 1/(gamma-1), gamma/(gamma-1)
   float gamma_f, gm1_f, r1_f, r2_f;
 };
@@ -52,6 +53,8 @@ inline void stage_args_derived(StageArgs& a) {
   a.sdx = a.dtx_scale / a.dx;
   a.sdy = a.dtx_scale / a.dy;
   a.sdz = a.dtx_scale / a.dz;
+  a.ryx = a.dx / a.dy;
+  a.rzx = a.dx / a.dz;
   a.gm1 = a.gamma - 1.0;
   a.r1 = 1.0 / (a.gamma - 1.0);
   a.r2 = a.gamma / (a.gamma - 1.0);

@@ -635,7 +635,7 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
   double* const Uhost = a.Uhost;
   const double* const Ubase = a.Ubase;
   const double* const U1 = a.U1;
-  const double dtx = ks.dtx, dty = ks.dty, glmf = ks.glmf;
+  const double dtx = ks.dtx, dty = ks.dty, glmf = ks.glmf, ryx = a.ryx;
   const bool iso = a.iso, rk2 = a.stage == 1 || a.time_type == OMHD_TIME_RK2, stage2 = a.stage == 2;
   int flip[4];
 #pragma unroll
@@ -653,6 +653,17 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
       const double* fx = m.FX + v * m.fxv + ty * m.fxr + tx;
       const double dF = fx[0] - fx[1];
       const double gm = m.FY[v * m.fyv + ty * TX + tx], gp = m.FY[v * m.fyv + (ty + 1) * TX + tx];
+      if constexpr (OMHD_FAST && sizeof(T) == 8) {
+        // rk.f90:26-35, :56-66 as U + dt/dx (dF + dx/dy dG): 4 (stage 1) or 5 FP64
+        // operations a variable instead of 5 or 8, as many roundings of the sum
+        const double ub = v == PS ? glmf * Ubase[v * N + c] : Ubase[v * N + c];
+        const double d = fma(ryx, gm - gp, dF);
+        if (rk2)
+          out[v] = fma(dtx, d, ub);
+        else
+          out[v] = half_exact(fma(dtx, d, ub + U1[v * N + c]));
+        continue;
+      }
       double d;
       if (iso)
         d = dtx * (dF + gm - gp);  // rk.f90:26-35 operation order

@@ -549,6 +549,14 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
       double out[NV];
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
+        if constexpr (OMHD_FAST && sizeof(T) == 8) {  // U + dt/dx (dF + dx/dy dG + dx/dz dH)
+          const double ub = v == PS ? glmf * a.Ubase[v * N + c] : a.Ubase[v * N + c];
+          const bool rk2 = a.stage == 1 || a.time_type == OMHD_TIME_RK2;
+          const double u0 = rk2 ? ub : ub + a.U1[v * N + c];
+          const double d = fma(dtx, fma(a.rzx, Fzp[v] - Fzc[v], fma(a.ryx, gm[v] - gp[v], acc[v])), u0);
+          out[v] = rk2 ? d : half_exact(d);
+          continue;
+        }
         double d;
         if (a.iso)
           d = dtx * (acc[v] + gm[v] - gp[v] + Fzp[v] - Fzc[v]);  // 3D_basic/rk.f90:26-35 order

@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_stage3d_pipe(const StageArgs a) {
   } else {
     // ======================= consumers =======================
     const int t = threadIdx.x - NP;
-    const double dtx = a.dtx_scale * dt / a.dx, dty = a.dtx_scale * dt / a.dy, dtz = a.dtx_scale * dt / a.dz;
+    const double dtx = a.dtx_scale * dt / a.dx;
     const double f1g = gamma - 1;
     for (int i = 0; i < nplanes; ++i) {
       const int p = k0 + i, b = i & 1;
@@ -469,17 +469,12 @@ __global__ void __launch_bounds__(NTOT, 1) k_stage3d_pipe(const StageArgs a) {
           const double gm = m.SLy[v * NYS + ty * TX + tx], gp = m.SLy[v * NYS + (ty + 1) * TX + tx];
           const double fzm = Fzm[v * NCELL + c], fzp = m.SLz[v * NZF + c];
           Fzm[v * NCELL + c] = fzp;  // face p+1/2 is the next plane's lower face
-          double d;
-          if (a.iso)
-            d = dtx * (acc + gm - gp + fzm - fzp);  // 3D_basic/rk.f90:26-35 order
-          else
-            d = dtx * acc + dty * (gm - gp) + dtz * (fzm - fzp);
-          double ub = a.Ubase[v * N + cc0];
-          if (v == PS) ub = glmf * ub;
-          if (a.stage == 1 || a.time_type == OMHD_TIME_RK2)
-            out[v] = ub + d;
-          else
-            out[v] = 0.5 * (ub + a.U1[v * N + cc0] + d);
+          // 3D_basic/rk.f90:26-35 as U + dt/dx (dF + dx/dy dG + dx/dz dH)
+          const double ub = v == PS ? glmf * a.Ubase[v * N + cc0] : a.Ubase[v * N + cc0];
+          const bool rk2 = a.stage == 1 || a.time_type == OMHD_TIME_RK2;
+          const double u0 = rk2 ? ub : ub + a.U1[v * N + cc0];
+          const double d = fma(dtx, fma(a.rzx, fzm - fzp, fma(a.ryx, gm - gp, acc)), u0);
+          out[v] = rk2 ? d : half_exact(d);
         }
         if (a.stage == 2) out[PS] = glmf * out[PS];
         int xt[3], yt[3], zt[3], xf[3], yf[3], zf[3], nxt = 1, nyt = 1, nzt = 1;

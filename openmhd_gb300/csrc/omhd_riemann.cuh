@@ -251,145 +251,168 @@ __device__ __forceinline__ void reconstruct_t(int type, T wm, T w0, T wp, T& lef
     reconstruct<T>(type, wm, w0, wp, left, right);
 }
 
-// HLLD intermediate (star) state of one side (flux_solver.f90:482-493 for L,
-// :496-507 for R, the same expressions with the side's values): side state
-// rho, normal / tangential velocities, tangential fields, wave speed a, total
-// energy E, total pressure pts, v.B, star density ros = rho*(a - un)/(a - aM)
-// and ie = 1/(a - aM); returns the star state's conserved variables in S and
-// its tangential velocities in v1, v2.
-template <class T, bool FAST, int vn, int vt1, int vt2, int bt1, int bt2, int mn, int mt1, int mt2>
-__device__ __forceinline__ void star_state(T ro, T un, T ut1, T ut2, T b1, T b2, T a, T E, T pts, T vB, T ros, T ie,
-                                           T aM, T pt, T Bn, T (&S)[NV], T& v1, T& v2) {
-  const T t = a - un;
-  const T f = rcp_<T, FAST>(ro * t * (a - aM) - Bn * Bn);
-  const T fb = f * (ro * (t * t) - Bn * Bn);  // B_t* = B_t fb, v_t* = v_t - B_t fv
-  const T fv = f * Bn * (aM - un);
-  S[bt1] = b1 * fb;
-  S[bt2] = b2 * fb;
-  v1 = ut1 - fv * b1;
-  v2 = ut2 - fv * b2;
-  S[RO] = ros;
-  S[EN] = divr_<T, FAST>((t * E - pts * un + pt * aM + Bn * (vB - aM * Bn - v1 * S[bt1] - v2 * S[bt2])), (a - aM), ie);
-  S[mn] = ros * aM;
-  S[mt1] = ros * v1;
-  S[mt2] = ros * v2;
-}
-
-// Per-side quantities of the FP64 HLLD solver (flux_solver.f90:359-401)
-// that both sides need: conserved normal momentum, normal momentum flux,
-// total pressure and the numerator of the fast speed squared,
-// cf^2 = num / (2 rho); the conserved energy and v.B (UE, vB) are filled in
-// by hlld_side_e for the sides whose star state or flux is built.
-struct HSide {
-  double B2, vB, Umn, UE, Fmn, pt, num;
+// The FP64 HLLD solver of the performance variant is written over a policy for
+// its plain products (those that no addition absorbs into a multiply-add, four in
+// ten of its operations): MulInt makes them on the integer pipes (mul_int), which
+// leaves a face 70-110 FP64-pipe operations instead of ~150-220; MulFp64 makes
+// them on the FP64 pipe.  A face whose operands mul_int does not take (infinite,
+// NaN, 2^511 or more) is solved again with MulFp64.
+struct MulInt {
+  bool bad = false;
+  __device__ __forceinline__ double operator()(double a, double b) { return mul_int(a, b, bad); }
+};
+struct MulFp64 {
+  static constexpr bool bad = false;
+  __device__ __forceinline__ double operator()(double a, double b) { return a * b; }
 };
 
-template <int DIR, int TAPE>
-__device__ __forceinline__ HSide hlld_side(const double (&S)[NV], double gamma, double r1, unsigned* code,
+// Per-side quantities of the FP64 HLLD solver (flux_solver.f90:359-401)
+// that both sides need: B^2, total pressure, q = pt - Bn^2 and the numerator of
+// the fast speed squared, cf^2 = num / (2 rho).  The conserved energy and v.B
+// (UE, vB) are filled in by hlld_side_e, the normal momentum (Umn) by
+// hlld_phys_flux, for the sides whose star state or flux is built.
+struct HSide {
+  double B2, pt, q, num, vB, UE, Umn;
+};
+
+template <int DIR, int TAPE, class M>
+__device__ __forceinline__ HSide hlld_side(const double (&S)[NV], double gamma, double gamma4, M& mul, unsigned* code,
                                            unsigned clamp_bit) {
-  constexpr int vn = VX + (DIR - 1) % 3, bn = BX + (DIR - 1) % 3;
+  constexpr int bn = BX + (DIR - 1) % 3, bt1 = BX + DIR % 3, bt2 = BX + (DIR + 1) % 3;
   HSide o;
-  o.B2 = S[BX] * S[BX] + S[BY] * S[BY] + S[BZ] * S[BZ];
-  o.vB = 0.0;
-  o.UE = 0.0;
-  o.Umn = S[RO] * S[vn];
-  o.pt = S[PR] + 0.5 * o.B2;
-  o.Fmn = o.Umn * S[vn] + o.pt - S[bn] * S[bn];  // rho vn^2 + pt - bn^2
-  const double f1 = gamma * S[PR], f2 = 4 * (S[bn] * S[bn]);
-  const double D = (f1 + o.B2) * (f1 + o.B2) - f1 * f2;
+  const double bn2 = mul(S[bn], S[bn]);
+  o.B2 = fma(S[bt2], S[bt2], fma(S[bt1], S[bt1], bn2));
+  o.vB = o.UE = o.Umn = 0.0;
+  o.pt = fma(0.5, o.B2, S[PR]);
+  o.q = o.pt - bn2;
+  const double f = fma(gamma, S[PR], o.B2);  // gamma p + B^2
+  const double D = fma(-mul(gamma4, S[PR]), bn2, mul(f, f));
   const bool cl = tape::decide<TAPE>(lt0_<double, true>(D), code, clamp_bit);  // fmax2(D, 0)
-  o.num = (f1 + o.B2) + sqrt_nr(cl ? 0.0 : D);
+  o.num = f + sqrt_nr(cl ? 0.0 : D);
   return o;
 }
 
 // conserved energy and v.B of one side (flux_solver.f90:360-362)
-__device__ __forceinline__ void hlld_side_e(const double (&S)[NV], double r1, HSide& o) {
-  const double v2 = S[VX] * S[VX] + S[VY] * S[VY] + S[VZ] * S[VZ];
-  o.vB = S[VX] * S[BX] + S[VY] * S[BY] + S[VZ] * S[BZ];
-  o.UE = 0.5 * (S[RO] * v2 + o.B2) + r1 * S[PR];
+template <class M>
+__device__ __forceinline__ void hlld_side_e(const double (&S)[NV], double r1, M& mul, HSide& o) {
+  const double v2 = fma(S[VZ], S[VZ], fma(S[VY], S[VY], mul(S[VX], S[VX])));
+  o.vB = fma(S[VZ], S[BZ], fma(S[VY], S[BY], mul(S[VX], S[BX])));
+  o.UE = fma(0.5, fma(S[RO], v2, o.B2), mul(r1, S[PR]));
 }
 
 // the physical flux of one side from its primitive state and HSide values
-template <int DIR>
-__device__ __forceinline__ void hlld_phys_flux(const double (&S)[NV], const HSide& h, double (&F)[NV]) {
+template <int DIR, class M>
+__device__ __forceinline__ void hlld_phys_flux(const double (&S)[NV], HSide& h, M& mul, double (&F)[NV]) {
   constexpr int vn = VX + (DIR - 1) % 3, vt1 = VX + DIR % 3, vt2 = VX + (DIR + 1) % 3;
   constexpr int bn = BX + (DIR - 1) % 3, bt1 = BX + DIR % 3, bt2 = BX + (DIR + 1) % 3;
   constexpr int mn = MX + (DIR - 1) % 3, mt1 = MX + DIR % 3, mt2 = MX + (DIR + 1) % 3;
+  h.Umn = mul(S[RO], S[vn]);
   F[RO] = h.Umn;
-  F[mn] = h.Fmn;
-  F[mt1] = h.Umn * S[vt1] - S[bn] * S[bt1];
-  F[mt2] = h.Umn * S[vt2] - S[bn] * S[bt2];
-  F[EN] = (h.UE + h.pt) * S[vn] - h.vB * S[bn];  // (E + pt) vn - (v.B) bn
-  F[bt1] = S[vn] * S[bt1] - S[bn] * S[vt1];
-  F[bt2] = S[vn] * S[bt2] - S[bn] * S[vt2];
+  F[mn] = fma(h.Umn, S[vn], h.q);  // rho vn^2 + pt - bn^2
+  F[mt1] = fma(h.Umn, S[vt1], -mul(S[bn], S[bt1]));
+  F[mt2] = fma(h.Umn, S[vt2], -mul(S[bn], S[bt2]));
+  F[EN] = fma(h.UE + h.pt, S[vn], -mul(h.vB, S[bn]));  // (E + pt) vn - (v.B) bn
+  F[bt1] = fma(S[vn], S[bt1], -mul(S[bn], S[vt1]));
+  F[bt2] = fma(S[vn], S[bt2], -mul(S[bn], S[vt2]));
   F[bn] = 0.0;
   F[PS] = 0.0;
+}
+
+// HLLD intermediate (star) state of one side (flux_solver.f90:482-493 for L,
+// :496-507 for R): t = a - un, rt = rho t, c = a - aM, ie = 1/c, du = aM - un,
+// total energy E, total pressure pts, v.B, star density ros; returns the star
+// state's conserved variables in S and its tangential velocities in v1, v2.
+template <int mn, int mt1, int mt2, int bt1, int bt2, class M>
+__device__ __forceinline__ void hlld_star(double un, double ut1, double ut2, double b1, double b2, double t, double rt,
+                                          double c, double ie, double du, double E, double pts, double vB, double ros,
+                                          double aM, double pt, double Bn, double Bn2, M& mul, double (&S)[NV],
+                                          double& v1, double& v2) {
+  const double f = rcp_nr(fma(rt, c, -Bn2));
+  const double fb = mul(f, fma(rt, t, -Bn2));  // B_t* = B_t fb, v_t* = v_t - B_t fv
+  const double fv = mul(mul(f, Bn), du);
+  S[bt1] = mul(b1, fb);
+  S[bt2] = mul(b2, fb);
+  v1 = fma(-fv, b1, ut1);
+  v2 = fma(-fv, b2, ut2);
+  S[RO] = ros;
+  const double w = fma(-v2, S[bt2], fma(-v1, S[bt1], fma(-aM, Bn, vB)));
+  S[EN] = mul(fma(Bn, w, fma(pt, aM, fma(-pts, un, mul(t, E)))), ie);
+  S[mn] = mul(ros, aM);
+  S[mt1] = mul(ros, v1);
+  S[mt2] = mul(ros, v2);
 }
 
 // HLLD flux of the FAST FP64 variant (flux_solver.f90:352-585, HLLC-G
 // fallback :447-476, GLM fluxes :580-581).  Same mathematics and decisions as
 // riemann_flux<double, DIR, FX_HLLD>; its work is cut to what the face's
-// region uses: per side only the quantities both sides need (the conserved
-// normal momentum and energy, the normal momentum flux, total pressure and
-// the fast-speed numerator); the HLL average only for rho, the normal momentum
-// and Bn (the tangential components serve the HLLC-G fallback alone); the
-// physical flux and the star state of the side s the region uses, from
-// side-selected inputs (the central region adds the other side's star state).
-template <int DIR, int TAPE>
-__device__ __forceinline__ void hlld_f64(const double (&L)[NV], const double (&R)[NV], double ch, double gamma,
-                                         double r1, double r2, double (&Fo)[NV], unsigned* code_io) {
+// region uses: per side only the quantities both sides need (total pressure and
+// the fast-speed numerator); of the HLL average only rho and the normal momentum
+// (their quotient aM) and Bn (the tangential components serve the HLLC-G fallback
+// alone); the physical flux and the star state of the side s the region uses,
+// from side-selected inputs (the central region adds the other side's star
+// state).
+template <int DIR, int TAPE, class M>
+__device__ __forceinline__ void hlld_f64_with(const double (&L)[NV], const double (&R)[NV], double ch, double gamma,
+                                              double r1, double (&Fo)[NV], unsigned& code_reg, M& mul) {
   using tape::decide;
-  unsigned code_reg = (TAPE == tape::kReplay) ? *code_io : 0u;
   unsigned* const code = &code_reg;
   constexpr int vn = VX + (DIR - 1) % 3, vt1 = VX + DIR % 3, vt2 = VX + (DIR + 1) % 3;
   constexpr int bn = BX + (DIR - 1) % 3, bt1 = BX + DIR % 3, bt2 = BX + (DIR + 1) % 3;
   constexpr int mn = MX + (DIR - 1) % 3, mt1 = MX + DIR % 3, mt2 = MX + (DIR + 1) % 3;
-  (void)r2;
-  HSide hL = hlld_side<DIR, TAPE>(L, gamma, r1, code, tape::kClampL);
-  HSide hR = hlld_side<DIR, TAPE>(R, gamma, r1, code, tape::kClampR);
+  const double gamma4 = 4 * gamma;
+  HSide hL = hlld_side<DIR, TAPE>(L, gamma, gamma4, mul, code, tape::kClampL);
+  HSide hR = hlld_side<DIR, TAPE>(R, gamma, gamma4, mul, code, tape::kClampR);
   // largest fast speed: cf^2 = num / (2 rho), numL/rhoL < numR/rhoR <=> numL*rhoR < numR*rhoL
-  const bool sr = decide<TAPE>(lt_<double, true>(hL.num * R[RO], hR.num * L[RO]), code, tape::kArSel);
-  const double cf = sqrt_ratio_<double, true>(sr ? hR.num : hL.num, 2 * (sr ? R[RO] : L[RO]));
+  const bool sr = decide<TAPE>(lt_<double, true>(mul(hL.num, R[RO]), mul(hR.num, L[RO])), code, tape::kArSel);
+  const double cn = sr ? hR.num : hL.num, cd = 2 * (sr ? R[RO] : L[RO]);
+  const double cnd = mul(cn, cd);
+  double cf;
+  if (pos_normal(cnd))
+    cf = mul(cn, rsqrt_nr(cnd));
+  else
+    cf = sqrt(cn / cd);
   const double aL = (decide<TAPE>(lt_<double, true>(R[vn], L[vn]), code, tape::kMinR) ? R[vn] : L[vn]) - cf;
   const double aR = (decide<TAPE>(lt_<double, true>(L[vn], R[vn]), code, tape::kMaxR) ? R[vn] : L[vn]) + cf;
   if (decide<TAPE>(ge0_<double, true>(aL), code, tape::kFL)) {
-    hlld_side_e(L, r1, hL);
-    hlld_phys_flux<DIR>(L, hL, Fo);
+    hlld_side_e(L, r1, mul, hL);
+    hlld_phys_flux<DIR>(L, hL, mul, Fo);
   } else if (decide<TAPE>(le0_<double, true>(aR), code, tape::kFR)) {
-    hlld_side_e(R, r1, hR);
-    hlld_phys_flux<DIR>(R, hR, Fo);
+    hlld_side_e(R, r1, mul, hR);
+    hlld_phys_flux<DIR>(R, hR, mul, Fo);
   } else {
-    // HLL average (:408-417) of rho, the normal momentum and Bn
-    const double f1 = rcp_nr(aR - aL);
+    // HLL average (:408-417): aM = Uh[mn]/Uh[rho], whose common factor
+    // 1/(aR - aL) cancels, and Bn
     const double tL = aL - L[vn], tR = aR - R[vn];
-    const double rtL = L[RO] * tL, rtR = R[RO] * tR;  // rho (a - vn) = a*rho - F[rho]
-    const double UhRO = f1 * (rtR - rtL);
-    const double Uhmn = f1 * ((aR * hR.Umn - hR.Fmn) - (aL * hL.Umn - hL.Fmn));
-    const double Ubn = f1 * (aR * R[bn] - aL * L[bn]);
-    const double aM = Uhmn * rcp_nr(UhRO);
-    const double pt = hL.pt + rtL * (aM - L[vn]);
-    const double ieL = rcp_nr(aL - aM), ieR = rcp_nr(aR - aM);
-    const double roL = rtL * ieL, roR = rtR * ieR;
+    const double rtL = mul(L[RO], tL), rtR = mul(R[RO], tR);  // rho (a - vn) = a*rho - F[rho]
+    const double f1 = rcp_nr(aR - aL);
+    const double Xro = rtR - rtL;
+    const double Xmn = fma(rtR, R[vn], -hR.q) - fma(rtL, L[vn], -hL.q);  // a*rho*vn - F[mn] = rho (a - vn) vn - q
+    const double Ubn = mul(f1, fma(aR, R[bn], -mul(aL, L[bn])));
+    const double aM = mul(Xmn, rcp_nr(Xro));
+    const double dL = aM - L[vn], dR = aM - R[vn];
+    const double pt = fma(rtL, dL, hL.pt);
+    const double cL = aM - aL, cR = aR - aM;
+    const double ieL = rcp_nr(-cL), ieR = rcp_nr(cR);
+    const double roL = mul(rtL, ieL), roR = mul(rtR, ieR);
     const bool bneg = decide<TAPE>(signbit(Ubn) != 0, code, tape::kBnNeg);
     const double aBn = (TAPE == tape::kNone) ? fabs(Ubn) : (bneg ? -Ubn : Ubn);
     // Alfven speeds aV = |Bn|/sqrt(rho*) enter the HLLC-G switch and the region
     // only through comparisons, which are made on squares (no square root
-    // unless the central states need sqrt(rho*)):
+    // unless the central states need sqrt(rho*)); c^2 rho* = c rho |a - vn|:
     //   aL >= aM - h aV_L  <=>  aM - aL <= 0  or  h^2 Bn^2 >= (aM - aL)^2 rho*_L
     //   aM + h aV_R >= aR  <=>  aR - aM <= 0  or  h^2 Bn^2 >= (aR - aM)^2 rho*_R
     const double hllg = 1.001;
-    const double Bn2 = Ubn * Ubn, hB2 = (hllg * hllg) * Bn2;
-    const double cL = aM - aL, cR = aR - aM;
-    if (decide<TAPE>(le0_<double, true>(cL) || !lt_<double, true>(hB2, (cL * cL) * roL) ||
-                         le0_<double, true>(cR) || !lt_<double, true>(hB2, (cR * cR) * roR),
+    const double Bn2 = mul(Ubn, Ubn), hB2 = mul(hllg * hllg, Bn2);
+    if (decide<TAPE>(le0_<double, true>(cL) || !lt_<double, true>(hB2, mul(cL, -rtL)) ||
+                         le0_<double, true>(cR) || !lt_<double, true>(hB2, mul(cR, rtR)),
                      code, tape::kG)) {
       // HLLC-G fallback :450-476 (rare): the tangential HLL components and
       // both physical fluxes
-      hlld_side_e(L, r1, hL);
-      hlld_side_e(R, r1, hR);
+      hlld_side_e(L, r1, mul, hL);
+      hlld_side_e(R, r1, mul, hR);
       double FL[NV], FR[NV];
-      hlld_phys_flux<DIR>(L, hL, FL);
-      hlld_phys_flux<DIR>(R, hR, FR);
+      hlld_phys_flux<DIR>(L, hL, mul, FL);
+      hlld_phys_flux<DIR>(R, hR, mul, FR);
       const double ULt1 = L[RO] * L[vt1], ULt2 = L[RO] * L[vt2], URt1 = R[RO] * R[vt1], URt2 = R[RO] * R[vt2];
       const double Uhmt1 = f1 * (aR * URt1 - aL * ULt1 - FR[mt1] + FL[mt1]);
       const double Uhmt2 = f1 * (aR * URt2 - aL * ULt2 - FR[mt2] + FL[mt2]);
@@ -398,11 +421,11 @@ __device__ __forceinline__ void hlld_f64(const double (&L)[NV], const double (&R
       const double f2 = aL * aR;
       Fo[bt1] = f1 * (aR * FL[bt1] - aL * FR[bt1] + f2 * (R[bt1] - L[bt1]));
       Fo[bt2] = f1 * (aR * FL[bt2] - aL * FR[bt2] + f2 * (R[bt2] - L[bt2]));
-      const double iUr = rcp_nr(UhRO);
+      const double iUr = rcp_nr(f1 * Xro);
       const double at1 = Uhmt1 * iUr, at2 = Uhmt2 * iUr;
-      const double enL = ((aL - L[vn]) * hL.UE - hL.pt * L[vn] + pt * aM +
+      const double enL = (tL * hL.UE - hL.pt * L[vn] + pt * aM +
                           Ubn * (hL.vB - aM * Ubn - at1 * Uhbt1 - at2 * Uhbt2)) * ieL;
-      const double enR = ((aR - R[vn]) * hR.UE - hR.pt * R[vn] + pt * aM +
+      const double enR = (tR * hR.UE - hR.pt * R[vn] + pt * aM +
                           Ubn * (hR.vB - aM * Ubn - at1 * Uhbt1 - at2 * Uhbt2)) * ieR;
       const double g1 = (TAPE != tape::kNone) ? (decide<TAPE>(signbit(aM) == 0, code, tape::kGLeft) ? 1.0 : 0.0)
                                               : 0.5 + fsign(0.5, aM);  // 0.5 + sign(0.5, aM)
@@ -416,10 +439,10 @@ __device__ __forceinline__ void hlld_f64(const double (&L)[NV], const double (&R
       // region (:482-572), then the side s whose state the flux uses
       //   aL1 = aM - aV_L >= 0  <=>  aM >= 0 and aM^2 rho*_L >= Bn^2
       //   aR1 = aM + aV_R <= 0  <=>  aM <= 0 and aM^2 rho*_R >= Bn^2
-      const double aM2 = aM * aM;
-      const bool sLs = decide<TAPE>(ge0_<double, true>(aM) && !lt_<double, true>(aM2 * roL, Bn2), code, tape::kLS);
+      const double aM2 = mul(aM, aM);
+      const bool sLs = decide<TAPE>(ge0_<double, true>(aM) && !lt_<double, true>(mul(aM2, roL), Bn2), code, tape::kLS);
       const bool sRs =
-          !sLs && decide<TAPE>(le0_<double, true>(aM) && !lt_<double, true>(aM2 * roR, Bn2), code, tape::kRS);
+          !sLs && decide<TAPE>(le0_<double, true>(aM) && !lt_<double, true>(mul(aM2, roR), Bn2), code, tape::kRS);
       const bool cen = !sLs && !sRs;
       const bool sR = sRs || (cen && !decide<TAPE>(ge0_<double, true>(aM), code, tape::kSSLeft));
       double Ss[NV];  // side primitive state
@@ -427,30 +450,29 @@ __device__ __forceinline__ void hlld_f64(const double (&L)[NV], const double (&R
       for (int v = 0; v < NV; ++v) Ss[v] = sR ? R[v] : L[v];
       HSide hs;
       hs.B2 = sR ? hR.B2 : hL.B2;
-      hs.Umn = sR ? hR.Umn : hL.Umn;
-      hs.Fmn = sR ? hR.Fmn : hL.Fmn;
       hs.pt = sR ? hR.pt : hL.pt;
-      hlld_side_e(Ss, r1, hs);
-      const double as = sR ? aR : aL;
+      hs.q = sR ? hR.q : hL.q;
+      hlld_side_e(Ss, r1, mul, hs);
+      const double as = sR ? aR : aL, ros = sR ? roR : roL;
       double S1[NV] = {}, vs1, vs2;
-      star_state<double, true, vn, vt1, vt2, bt1, bt2, mn, mt1, mt2>(
-          Ss[RO], Ss[vn], Ss[vt1], Ss[vt2], Ss[bt1], Ss[bt2], as, hs.UE, hs.pt, hs.vB, sR ? roR : roL,
-          sR ? ieR : ieL, aM, pt, Ubn, S1, vs1, vs2);
+      hlld_star<mn, mt1, mt2, bt1, bt2>(Ss[vn], Ss[vt1], Ss[vt2], Ss[bt1], Ss[bt2], sR ? tR : tL, sR ? rtR : rtL,
+                                        sR ? cR : -cL, sR ? ieR : ieL, sR ? dR : dL, hs.UE, hs.pt, hs.vB, ros, aM, pt,
+                                        Ubn, Bn2, mul, S1, vs1, vs2);
       double Fs[NV], Us[NV];  // the side's physical flux and state (conserved MX..EN, primitive rho and B)
-      hlld_phys_flux<DIR>(Ss, hs, Fs);
+      hlld_phys_flux<DIR>(Ss, hs, mul, Fs);
       Us[mn] = hs.Umn;
-      Us[mt1] = Ss[RO] * Ss[vt1];
-      Us[mt2] = Ss[RO] * Ss[vt2];
+      Us[mt1] = mul(Ss[RO], Ss[vt1]);
+      Us[mt2] = mul(Ss[RO], Ss[vt2]);
       Us[EN] = hs.UE;
       Us[RO] = Ss[RO];
       Us[bt1] = Ss[bt1];
       Us[bt2] = Ss[bt2];
       if (!cen) {  // F(L*) :514-519 / F(R*) :522-527
 #pragma unroll
-        for (int v = MX; v <= EN; ++v) Fo[v] = as * (S1[v] - Us[v]) + Fs[v];
-        Fo[RO] = as * (S1[RO] - Us[RO]) + Fs[RO];
-        Fo[bt1] = as * (S1[bt1] - Us[bt1]) + Fs[bt1];
-        Fo[bt2] = as * (S1[bt2] - Us[bt2]) + Fs[bt2];
+        for (int v = MX; v <= EN; ++v) Fo[v] = fma(as, S1[v] - Us[v], Fs[v]);
+        Fo[RO] = fma(as, S1[RO] - Us[RO], Fs[RO]);
+        Fo[bt1] = fma(as, S1[bt1] - Us[bt1], Fs[bt1]);
+        Fo[bt2] = fma(as, S1[bt2] - Us[bt2], Fs[bt2]);
       } else {  // central states :533-572, symmetric in (s, o); sigma = +1 for s = L, -1 for s = R
         double So[NV];  // the other side's primitive state
 #pragma unroll
@@ -458,41 +480,81 @@ __device__ __forceinline__ void hlld_f64(const double (&L)[NV], const double (&R
         HSide ho;
         ho.B2 = sR ? hL.B2 : hR.B2;
         ho.pt = sR ? hL.pt : hR.pt;
-        hlld_side_e(So, r1, ho);
+        hlld_side_e(So, r1, mul, ho);
+        const double roo = sR ? roL : roR;
         double O1[NV] = {}, vo1, vo2;
-        star_state<double, true, vn, vt1, vt2, bt1, bt2, mn, mt1, mt2>(
-            So[RO], So[vn], So[vt1], So[vt2], So[bt1], So[bt2], sR ? aL : aR, ho.UE, ho.pt, ho.vB,
-            sR ? roL : roR, sR ? ieL : ieR, aM, pt, Ubn, O1, vo1, vo2);
-        const double ros = sR ? roR : roL, roo = sR ? roL : roR;
-        const double rsS = rsqrt_nr(ros), rsO = rsqrt_nr(roo);  // 1/sqrt(rho*) of s and o
-        const double rss = ros * rsS, rso = roo * rsO;          // sqrt(rho*) of s and o
+        hlld_star<mn, mt1, mt2, bt1, bt2>(So[vn], So[vt1], So[vt2], So[bt1], So[bt2], sR ? tL : tR, sR ? rtL : rtR,
+                                          sR ? -cL : cR, sR ? ieL : ieR, sR ? dL : dR, ho.UE, ho.pt, ho.vB, roo, aM, pt,
+                                          Ubn, Bn2, mul, O1, vo1, vo2);
+        const double rsS = rsqrt_nr(ros), rsO = rsqrt_nr(roo);      // 1/sqrt(rho*) of s and o
+        const double rss = mul(ros, rsS), rso = mul(roo, rsO);      // sqrt(rho*) of s and o
         const double fc = rcp_nr(rss + rso);
         const double f2 = (TAPE == tape::kNone) ? fsign(1.0, Ubn) : (bneg ? -1.0 : 1.0);
         const double f2s = sR ? -f2 : f2;
-        double U2[NV];
-        const double at1 = fc * (rss * vs1 + rso * vo1 + (O1[bt1] - S1[bt1]) * f2s);
-        const double at2 = fc * (rss * vs2 + rso * vo2 + (O1[bt2] - S1[bt2]) * f2s);
-        U2[bt1] = fc * (rss * O1[bt1] + rso * S1[bt1] + rss * rso * (vo1 - vs1) * f2s);
-        U2[bt2] = fc * (rss * O1[bt2] + rso * S1[bt2] + rss * rso * (vo2 - vs2) * f2s);
-        U2[RO] = ros;
-        U2[EN] = S1[EN] - rss * (vs1 * S1[bt1] + vs2 * S1[bt2] - at1 * U2[bt1] - at2 * U2[bt2]) * f2s;
-        U2[mn] = ros * aM;
-        U2[mt1] = ros * at1;
-        U2[mt2] = ros * at2;
-        const double as1 = sR ? aM + aBn * rsS : aM - aBn * rsS;  // aR1 = aM + aV_R, aL1 = aM - aV_L
-#pragma unroll
-        for (int v = MX; v <= EN; ++v) Fo[v] = as1 * U2[v] - (as1 - as) * S1[v] - as * Us[v] + Fs[v];
-        Fo[RO] = as1 * U2[RO] - (as1 - as) * S1[RO] - as * Us[RO] + Fs[RO];
-        Fo[bt1] = as1 * U2[bt1] - (as1 - as) * S1[bt1] - as * Us[bt1] + Fs[bt1];
-        Fo[bt2] = as1 * U2[bt2] - (as1 - as) * S1[bt2] - as * Us[bt2] + Fs[bt2];
+        const double rssf = copysign(rss, f2s), rr = mul(rssf, rso);  // rss f2s, rss rso f2s
+        const double at1 = mul(fc, fma(f2s, O1[bt1] - S1[bt1], fma(rss, vs1, mul(rso, vo1))));
+        const double at2 = mul(fc, fma(f2s, O1[bt2] - S1[bt2], fma(rss, vs2, mul(rso, vo2))));
+        const double U2b1 = mul(fc, fma(rr, vo1 - vs1, fma(rss, O1[bt1], mul(rso, S1[bt1]))));
+        const double U2b2 = mul(fc, fma(rr, vo2 - vs2, fma(rss, O1[bt2], mul(rso, S1[bt2]))));
+        const double w = fma(-at2, U2b2, fma(-at1, U2b1, fma(vs2, S1[bt2], mul(vs1, S1[bt1]))));
+        const double U2en = fma(-rssf, w, S1[EN]);
+        const double as1 = fma(sR ? aBn : -aBn, rsS, aM);  // aR1 = aM + aV_R, aL1 = aM - aV_L
+        const double das = as1 - as;
+        // rho* and rho* aM are the same in the star and central states
+        Fo[RO] = fma(as, ros - Us[RO], Fs[RO]);
+        Fo[mn] = fma(as, S1[mn] - Us[mn], Fs[mn]);
+        Fo[mt1] = fma(as1, mul(ros, at1), fma(-das, S1[mt1], fma(-as, Us[mt1], Fs[mt1])));
+        Fo[mt2] = fma(as1, mul(ros, at2), fma(-das, S1[mt2], fma(-as, Us[mt2], Fs[mt2])));
+        Fo[EN] = fma(as1, U2en, fma(-das, S1[EN], fma(-as, Us[EN], Fs[EN])));
+        Fo[bt1] = fma(as1, U2b1, fma(-das, S1[bt1], fma(-as, Us[bt1], Fs[bt1])));
+        Fo[bt2] = fma(as1, U2b2, fma(-das, S1[bt2], fma(-as, Us[bt2], Fs[bt2])));
       }
     }
   }
   // GLM fluxes :580-581, the halving folded into the (exact) half speeds
   const double hch = 0.5 * ch, hch2 = 0.5 * (ch * ch);
-  Fo[bn] = 0.5 * (L[PS] + R[PS]) - hch * (R[bn] - L[bn]);
-  Fo[PS] = hch2 * (L[bn] + R[bn]) - hch * (R[PS] - L[PS]);
-  if constexpr (TAPE == tape::kRecord) *code_io = code_reg;
+  Fo[bn] = fma(0.5, L[PS] + R[PS], -mul(hch, R[bn] - L[bn]));
+  Fo[PS] = fma(hch2, L[bn] + R[bn], -mul(hch, R[PS] - L[PS]));
+}
+
+// the same face with FP64-pipe products; out of line: it is entered for operands
+// outside mul_int's range only, and the inlined solver keeps its registers
+template <int DIR, int TAPE>
+__device__ __noinline__ void hlld_f64_wide_range(const double* LR, double ch, double gamma, double r1, double* F,
+                                                 unsigned* code) {
+  double L[NV], R[NV], Fo[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    L[v] = LR[v];
+    R[v] = LR[NV + v];
+  }
+  MulFp64 mul;
+  unsigned c = *code;
+  hlld_f64_with<DIR, TAPE>(L, R, ch, gamma, r1, Fo, c, mul);
+  *code = c;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) F[v] = Fo[v];
+}
+
+template <int DIR, int TAPE>
+__device__ __forceinline__ void hlld_f64(const double (&L)[NV], const double (&R)[NV], double ch, double gamma,
+                                         double r1, double (&Fo)[NV], unsigned* code_io) {
+  unsigned code = (TAPE == tape::kReplay) ? *code_io : 0u;
+  MulInt mul;
+  hlld_f64_with<DIR, TAPE>(L, R, ch, gamma, r1, Fo, code, mul);
+  if (mul.bad) {
+    double LR[2 * NV], F[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      LR[v] = L[v];
+      LR[NV + v] = R[v];
+    }
+    code = (TAPE == tape::kReplay) ? *code_io : 0u;
+    hlld_f64_wide_range<DIR, TAPE>(LR, ch, gamma, r1, F, &code);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) Fo[v] = F[v];
+  }
+  if constexpr (TAPE == tape::kRecord) *code_io = code;
 }
 
 // Numerical flux across one face (2D_basic/flux_solver.f90):
@@ -508,7 +570,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
                                              T r2, T (&Fo)[NV], unsigned* code_io = nullptr) {
   using tape::decide;
   if constexpr (FAST && sizeof(T) == 8 && TYPE == FX_HLLD) {
-    hlld_f64<DIR, TAPE>(L, R, ch, gamma, r1, r2, Fo, code_io);
+    hlld_f64<DIR, TAPE>(L, R, ch, gamma, r1, Fo, code_io);
     return;
   }
   // the face's decision word lives in a register here; read from / written to
@@ -846,13 +908,31 @@ __device__ __forceinline__ void u2v_cell(const double (&u)[NV], double f1g, floa
   }
   const double r = u[RO];
   const double mx = u[MX], my = u[MY], mz = u[MZ];
-  const double ir = rcp_<double, FAST>(r);  // one reciprocal for the three velocities
-  const double vx = divr_<double, FAST>(mx, r, ir), vy = divr_<double, FAST>(my, r, ir),
-               vz = divr_<double, FAST>(mz, r, ir);  // u2v.f90:24
-  const double rv2 = vx * mx + vy * my + vz * mz;
   const double bx = u[BX], by = u[BY], bz = u[BZ];
-  const double B2 = bx * bx + by * by + bz * bz;
-  const double p = f1g * (u[EN] - 0.5 * (rv2 + B2));  // u2v.f90:27
+  const double ir = rcp_<double, FAST>(r);  // one reciprocal for the three velocities
+  double vx, vy, vz, p;
+  if constexpr (FAST && sizeof(T) == 8) {  // the plain products on the integer pipes, as in the Riemann solver
+    auto recover = [&](auto& mul) {
+      vx = mul(mx, ir);
+      vy = mul(my, ir);
+      vz = mul(mz, ir);
+      const double e2 = fma(vz, mz, fma(vy, my, mul(vx, mx))) + fma(bz, bz, fma(by, by, mul(bx, bx)));
+      p = mul(f1g, fma(-0.5, e2, u[EN]));
+    };
+    MulInt mi;
+    recover(mi);
+    if (mi.bad) {
+      MulFp64 mf;
+      recover(mf);
+    }
+  } else {
+    vx = divr_<double, FAST>(mx, r, ir);
+    vy = divr_<double, FAST>(my, r, ir);
+    vz = divr_<double, FAST>(mz, r, ir);  // u2v.f90:24
+    const double rv2 = vx * mx + vy * my + vz * mz;
+    const double B2 = bx * bx + by * by + bz * bz;
+    p = f1g * (u[EN] - 0.5 * (rv2 + B2));  // u2v.f90:27
+  }
   w[VX] = to_face<T>(vx);
   w[VY] = to_face<T>(vy);
   w[VZ] = to_face<T>(vz);

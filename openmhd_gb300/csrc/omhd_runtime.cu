@@ -189,6 +189,18 @@ __global__ void k_fastmath_probe(const double* __restrict__ x, long long n, doub
   }
 }
 
+// mul_int(a, b), whether it refuses the operands (1.0) and half_exact(a): three
+// planes of n values
+__global__ void k_mul_probe(const double* __restrict__ a, const double* __restrict__ b, long long n,
+                            double* __restrict__ out) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    bool bad = false;
+    out[i] = mul_int(a[i], b[i], bad);
+    out[n + i] = bad ? 1.0 : 0.0;
+    out[2 * n + i] = half_exact(a[i]);
+  }
+}
+
 __global__ void k_convert_probe(const double* __restrict__ xd, float* __restrict__ nd, const float* __restrict__ xf,
                                 double* __restrict__ wf, long long n) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -256,6 +268,25 @@ int omhd_probe_fastmath(const double* x, long long n, double* out) {
   k_fastmath_probe<<<(unsigned)blocks, 256>>>(x, n, out);
   if (cuda_status(cudaGetLastError(), "fast-math probe launch")) return OMHD_CUDA_ERR;
   return cuda_status(cudaDeviceSynchronize(), "fast-math probe");
+}
+
+int omhd_probe_mul(const double* a, const double* b, long long n, double* out) {
+  if (!a || !b || !out || n < 0) return OMHD_BAD_ARG;
+  if (n == 0) return OMHD_OK;
+  const void* ptrs[3] = {a, b, out};
+  for (const void* p : ptrs) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeDevice) {
+      cudaGetLastError();
+      set_host_error(OMHD_BAD_ARG, 0, 0, 0, 0.0, "product probe: all three arrays must be device memory");
+      return OMHD_BAD_ARG;
+    }
+  }
+  long long blocks = (n + 255) / 256;
+  if (blocks > 4096) blocks = 4096;
+  k_mul_probe<<<(unsigned)blocks, 256>>>(a, b, n, out);
+  if (cuda_status(cudaGetLastError(), "product probe launch")) return OMHD_CUDA_ERR;
+  return cuda_status(cudaDeviceSynchronize(), "product probe");
 }
 
 int omhd_probe_convert(const double* xd, float* nd, const float* xf, double* wf, long long n) {
