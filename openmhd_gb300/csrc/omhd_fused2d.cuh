@@ -145,6 +145,7 @@ struct StageScalars {
   double glmf;        // GLM damping factor of the step (glm_ss2.f90:27)
   double dtx, dty;    // dtx_scale * dt / dx and / dy (rk.f90:22)
   T ch, gam, r1, r2;  // GLM speed, gamma, 1/(gamma-1), gamma/(gamma-1) (flux_solver.f90:38-39)
+  float known;        // CFL speed found so far in this stage (stage 2, cfl_known)
 };
 template <class T>
 __device__ __forceinline__ void stage_scalars(const StageArgs& a, const StepState* st, StageScalars<T>& k) {
@@ -158,6 +159,7 @@ __device__ __forceinline__ void stage_scalars(const StageArgs& a, const StepStat
     k.dty = a.dtx_scale * dt / a.dy;
   }
   k.ch = to_face<T>(st->ch);
+  k.known = a.stage == 2 ? cfl_known(st) : 0.0f;
   if constexpr (sizeof(T) == 4) {
     k.gam = a.gamma_f;
     k.r1 = a.r1_f;
@@ -617,10 +619,11 @@ __device__ __forceinline__ void phase_flux(const StageArgs& a, int bxi, int byi,
 }
 
 // phase D: update, ghost fill, GLM, CFL of the tile's cells t, t+n, ...;
-// returns this thread's largest CFL speed (stage 2) or 0
+// returns this thread's largest CFL speed (stage 2) of the cells that may hold the
+// grid's maximum, given that it is known or more; or 0
 template <class T, class G>
 __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t,
-                                               int n, const StageScalars<T>& ks) {
+                                               int n, const StageScalars<T>& ks, float known) {
   constexpr int TX = G::TX, TY = G::TY;
   const int ix = a.ix, jx = a.jx;
   const size_t N = (size_t)ix * jx;
@@ -628,6 +631,7 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
   const bool perx = a.bc_kind[0] == OMHD_BC_PERIODIC, pery = a.bc_kind[2] == OMHD_BC_PERIODIC;
   const double gamma = a.gamma;
   const double f1g = a.gm1;
+  const float gamma_f = a.gamma_f, gm1_f = a.gm1_f;
   // the argument block may live in global memory (ensembles), where a store to
   // the state could alias it: every pointer and scalar used in the loop is
   // read once, here
@@ -700,7 +704,8 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
         }
       }
 
-    if (stage2) {  // set_dt.f90:27-37 on the new state
+    // set_dt.f90:27-37 on the new state
+    if (stage2 && !(OMHD_FAST && known > 0.0f && cfl_upper<2>(out, gamma_f, gm1_f) < known)) {
       const double ro = out[RO];
       const double iro = rcp_<double, OMHD_FAST, sizeof(T) == 4>(ro);  // one reciprocal for the three velocities
       const double vx = divr_<double, OMHD_FAST>(out[MX], ro, iro), vy = divr_<double, OMHD_FAST>(out[MY], ro, iro),
@@ -737,7 +742,7 @@ __device__ __forceinline__ double stage2d_tile(const StageArgs& a, int bxi, int 
   }
   phase_flux<T, FLUX, G, TAPE>(a, bxi, byi, m, tid, G::NT, ks);
   __syncthreads();
-  return phase_update<T, G>(a, bxi, byi, m, tid, G::NT, ks);
+  return phase_update<T, G>(a, bxi, byi, m, tid, G::NT, ks, ks.known);
 }
 
 // one CTA per tile of one grid
@@ -905,9 +910,11 @@ __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
       const int b = i & 1;
       const TileMem<double> m = pipe_mem(smem_raw, b);
       named_bar_sync(kPipeBarFull + b, NTOT);
+      const float known = a.stage == 2 ? cfl_known(st) : 0.0f;
       phase_flux<double, FLUX, G, TAPE>(a, w % ntx, w / ntx, m, t, NC, ks);
       named_bar_sync(kPipeBarCons, NC);
-      const double v = phase_update<double, G>(a, w % ntx, w / ntx, m, t, NC, ks);
+      const double v = phase_update<double, G>(a, w % ntx, w / ntx, m, t, NC, ks, known);
+      if (a.stage == 2) cfl_publish(st, v, known);
       vmax = lt_<double, OMHD_FAST>(vmax, v) ? v : vmax;
       if (i + 2 < nmine) {  // the producers refill buffer b for tile i+2
         __threadfence_block();

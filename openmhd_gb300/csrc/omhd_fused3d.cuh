@@ -285,6 +285,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
 
   for (int k = lead_in ? k0 - 1 : k0; k <= k1; ++k) {
     const bool lead = k < k0;  // only the z face k+1/2 (uniform over the CTA)
+    const float known = OMHD_FAST && a.stage == 2 ? cfl_known(st) : 0.0f;  // read a plane ahead of its use
     // Three CTA barriers per plane (plus one where a wall fix is needed).  The
     // ring slot of plane k+2 held plane k-2, whose last readers (the resistive
     // terms of plane k-1) finished before the previous plane's flux barrier;
@@ -590,7 +591,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
               if (a.Uhost) a.Uhost[v * N + cc] = o;  // result straight to host memory
             }
           }
-      if (a.stage == 2) {  // 3D_basic/set_dt.f90:27-43 on the new state
+      // 3D_basic/set_dt.f90:27-43 on the new state
+      if (a.stage == 2 && !(OMHD_FAST && known > 0.0f && cfl_upper<3>(out, a.gamma_f, a.gm1_f) < known)) {
         const double ro = out[RO];
         const double iro = rcp_<double, OMHD_FAST, sizeof(T) == 4>(ro);  // one reciprocal for the three velocities
         const double vx = divr_<double, OMHD_FAST>(out[MX], ro, iro), vy = divr_<double, OMHD_FAST>(out[MY], ro, iro), vz = divr_<double, OMHD_FAST>(out[MZ], ro, iro);
@@ -606,6 +608,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
         double s = lt_<double, OMHD_FAST>(sx, sy) ? sy : sx;
         s = lt_<double, OMHD_FAST>(s, sz) ? sz : s;
         vloc = lt_<double, OMHD_FAST>(s, vloc) ? vloc : s;
+        if (OMHD_FAST) cfl_publish(st, s, known);
       }
     }
 #pragma unroll

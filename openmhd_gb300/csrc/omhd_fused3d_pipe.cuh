@@ -345,6 +345,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_stage3d_pipe(const StageArgs a) {
     const double dtx = a.dtx_scale * dt / a.dx;
     const double f1g = gamma - 1;
     for (int i = 0; i < nplanes; ++i) {
+      const float known = a.stage == 2 ? cfl_known(st) : 0.0f;
       const int p = k0 + i, b = i & 1;
       const Buf m = buf_at(bufbase + (size_t)b * BUF);
       if (t < NOWN)
@@ -497,7 +498,8 @@ __global__ void __launch_bounds__(NTOT, 1) k_stage3d_pipe(const StageArgs a) {
                 if (a.Uhost) a.Uhost[v * N + cc] = o;  // result straight to host memory
               }
             }
-        if (a.stage == 2) {  // 3D_basic/set_dt.f90:27-43 on the new state
+        // 3D_basic/set_dt.f90:27-43 on the new state
+        if (a.stage == 2 && !(known > 0.0f && cfl_upper<3>(out, a.gamma_f, a.gm1_f) < known)) {
           const double ro = out[RO];
           const double iro = rcp_<double, true>(ro);
           const double vx = divr_<double, true>(out[MX], ro, iro), vy = divr_<double, true>(out[MY], ro, iro),
@@ -514,6 +516,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_stage3d_pipe(const StageArgs a) {
           double s = lt_<double, true>(sx, sy) ? sy : sx;
           s = lt_<double, true>(s, sz) ? sz : s;
           vmax = lt_<double, true>(s, vmax) ? vmax : s;
+          cfl_publish(st, s, known);
         }
       }
       if (i + 2 < nplanes) {  // the producers refill buffer b for plane p+2

@@ -954,4 +954,46 @@ __device__ __forceinline__ T fast_speed(T f1, T B2, T bd, T ro) {
   return sqrt_ratio_<T, FAST, FPIPE>((f1 + B2) + sqrt_<T, FAST, FPIPE>(lt0_<T, FAST>(D) ? T(0) : D), 2 * ro);
 }
 
+// ---------------------------------------------------------------------------
+// The CFL maximum without most of its FP64 work.  set_dt needs the largest
+// |v| + fast speed of the grid, ~45 FP64 operations a cell with two or three
+// square roots; a binary32 upper bound of that speed, ~90 instructions of the
+// idle pipes, tells whether the cell can hold the maximum at all.  Only a cell
+// whose bound reaches a speed already found (known: a lower bound of the grid's
+// maximum, from StepState::vmax_acc, where every CTA publishes what it found) is
+// evaluated in FP64, so the maximum is the same double, whatever the order.
+// ---------------------------------------------------------------------------
+// |x| cut to binary32: 0 below 2^-126, infinity from 2^128 (and for NaN)
+__device__ __forceinline__ float magnitude_f32(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu, lo = (unsigned)__double2loint(x);
+  const unsigned f = __funnelshift_l(lo, hi - 0x38000000u, 3);
+  return __uint_as_float(hi < 0x38100000u ? 0u : (hi >= 0x47f00000u ? 0x7f800000u : f));
+}
+
+// An upper bound, within ~1e-4, of |v| + fast speed over the ND axes of a cell with
+// conserved variables u.  Rounding enters through the pressure (a difference of
+// energies: bounded by 2^-18 of their sum) and the discriminant (2^-18 of its
+// first term), both added; the rest is relative, 2^-14 covers it.  Infinity (no
+// statement) for a non-positive density or energy and outside [2^-60, 2^60].
+template <int ND>
+__device__ __forceinline__ float cfl_upper(const double (&u)[NV], float gamma, float gm1) {
+  const float r = magnitude_f32(u[RO]), e = magnitude_f32(u[EN]);
+  const float m[3] = {magnitude_f32(u[MX]), magnitude_f32(u[MY]), magnitude_f32(u[MZ])};
+  const float b[3] = {magnitude_f32(u[BX]), magnitude_f32(u[BY]), magnitude_f32(u[BZ])};
+  const float ir = __fdividef(1.0f, r);
+  const float B2 = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
+  const float ke = 0.5f * ((m[0] * m[0] + m[1] * m[1] + m[2] * m[2]) * ir + B2);
+  const float f1 = gamma * (gm1 * (fmaxf(e - ke, 0.0f) + 0x1p-18f * (e + ke)));
+  const float n0 = f1 + B2, n2 = n0 * n0;
+  float s = 0.0f;
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    const float D = fmaxf(n2 - 4.0f * f1 * (b[d] * b[d]), 0.0f) + 0x1p-18f * n2;
+    s = fmaxf(s, m[d] * ir + sqrtf(0.5f * ir * (n0 + sqrtf(D))));
+  }
+  const bool fine = r >= 0x1p-60f && r <= 0x1p60f && n0 >= 0x1p-60f && n0 <= 0x1p60f && e <= 0x1p60f &&
+                    __double2hiint(u[RO]) >= 0 && __double2hiint(u[EN]) >= 0;
+  return fine ? s * (1.0f + 0x1p-14f) : __int_as_float(0x7f800000);
+}
+
 }  // namespace omhd

@@ -184,6 +184,16 @@ __device__ __forceinline__ double cell_cfl_speed(const double (&u)[NV], double g
   return sp;
 }
 
+// v = max(v, CFL speed of the cell), the speed evaluated only if its binary32 bound
+// reaches what is known of the maximum
+__device__ __forceinline__ void cell_cfl_max(const double (&u)[NV], double gamma, float gamma_f, float gm1_f, int nd,
+                                             StepState* st, float known, double& v) {
+  if (known > 0.0f && (nd == 3 ? cfl_upper<3>(u, gamma_f, gm1_f) : cfl_upper<2>(u, gamma_f, gm1_f)) < known) return;
+  const double s = cell_cfl_speed(u, gamma, nd);
+  v = fmax2(s, v);
+  cfl_publish(st, s, known);
+}
+
 // CFL speed of the current state (set_dt.f90:27-52) + device step planning
 __global__ void k_init_cfl(const double* __restrict__ U, int ix, int jx, int kx, int nd, double gamma,
                            StepState* st, DevError* err, StepConsts sc) {
@@ -191,15 +201,18 @@ __global__ void k_init_cfl(const double* __restrict__ U, int ix, int jx, int kx,
   const int ni = ix - 2, nj = jx - 2, nk = (nd == 3) ? kx - 2 : 1;
   const long long total = (long long)ni * nj * nk;
   const size_t n = (size_t)ix * jx * kx;
+  const float gamma_f = (float)gamma, gm1_f = (float)(gamma - 1);
   double v = 0.0;
+  float known = 0.0f;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
+    known = fmaxf(known, cfl_known(st));
     const int i = 1 + (int)(t % ni), j = 1 + (int)((t / ni) % nj), k = (nd == 3 ? 1 : 0) + (int)(t / ((long long)ni * nj));
     const size_t c = (size_t)i + (size_t)ix * ((size_t)j + (size_t)jx * k);
     double u[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) u[q] = U[q * n + c];
-    v = fmax2(cell_cfl_speed(u, gamma, nd), v);
+    cell_cfl_max(u, gamma, gamma_f, gm1_f, nd, st, known, v);
   }
   const double bm = block_max_pos(v, red32);
   reduce_and_finalize(st, sc, err, bm, gridDim.x, 0);
@@ -213,7 +226,9 @@ __global__ void k_upload_cfl(const double* __restrict__ Uh, double* __restrict__
                              double gamma, StepState* st, DevError* err, StepConsts sc) {
   __shared__ double red32[32];
   const size_t n = (size_t)ix * jx * kx;
+  const float gamma_f = (float)gamma, gm1_f = (float)(gamma - 1);
   double v = 0.0;
+  float known = 0.0f;
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
     double u[NV];
 #pragma unroll
@@ -223,7 +238,10 @@ __global__ void k_upload_cfl(const double* __restrict__ Uh, double* __restrict__
     }
     const int i = (int)(c % ix), j = (int)((c / ix) % jx), k = (int)(c / ((size_t)ix * jx));
     const bool interior = i >= 1 && i <= ix - 2 && j >= 1 && j <= jx - 2 && (nd != 3 || (k >= 1 && k <= kx - 2));
-    if (interior) v = fmax2(cell_cfl_speed(u, gamma, nd), v);
+    if (interior) {
+      known = fmaxf(known, cfl_known(st));
+      cell_cfl_max(u, gamma, gamma_f, gm1_f, nd, st, known, v);
+    }
   }
   const double bm = block_max_pos(v, red32);
   reduce_and_finalize(st, sc, err, bm, gridDim.x, 0);

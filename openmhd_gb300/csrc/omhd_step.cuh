@@ -69,6 +69,27 @@ __device__ __forceinline__ void finalize_step(StepState* s, const StepConsts& c,
   plan_next_step(s, c, vmax, err);
 }
 
+// Lower bound, in binary32, of the grid's largest CFL speed: what the stage's CTAs
+// have published so far (0 when nothing is, or when it is below 2^-40: then every
+// cell is evaluated).
+__device__ __forceinline__ float cfl_known(const StepState* s) {
+  const unsigned long long b = *(const volatile unsigned long long*)&s->vmax_acc;
+  const unsigned hi = (unsigned)(b >> 32);
+  if (hi < 0x3d700000u || hi >= 0x47f00000u) return 0.0f;
+  return __uint_as_float(__funnelshift_l((unsigned)b, hi - 0x38000000u, 3));
+}
+
+// Publishes the calling lanes' largest speed if it raises what they knew (one
+// atomic per warp at most; the end-of-stage reduction remains the authority).
+__device__ __forceinline__ void cfl_publish(StepState* s, double v, float known) {
+  const unsigned mask = __activemask();
+  const unsigned hi = magnitude_f32(v) > known ? (unsigned)__double2hiint(v) : 0u;
+  const unsigned top = __reduce_max_sync(mask, hi);
+  if (top == 0u || top > 0x7ff00000u) return;
+  const unsigned who = __ballot_sync(mask, hi == top);
+  if ((int)(threadIdx.x & 31) == __ffs(who) - 1) atomic_max_pos_double(&s->vmax_acc, v);
+}
+
 // warp + block max of non-negative doubles; result valid in thread 0.  For
 // non-negative doubles the integer order of the bit patterns is the numeric
 // order, so the max runs on the integer pipe (a floating-point compare holds
