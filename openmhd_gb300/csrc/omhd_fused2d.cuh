@@ -193,11 +193,11 @@ __device__ __forceinline__ TileMem<T> tile_mem_separate(unsigned char* smem_raw)
 // the halo, so that the box starts on an even x), instead of in global memory.
 template <class T, class G, bool STAGED = false>
 __device__ __forceinline__ void phase_load(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t, int n,
-                                           double glmf, const double* S = nullptr) {
-  constexpr int TX = G::TX, TY = G::TY, RX = G::RX, RY = G::RY, PL = RX * RY;
+                                           double glmf, const double* S = nullptr, const int ty = G::TY) {
+  constexpr int TX = G::TX, RX = G::RX, RY = G::RY, PL = RX * RY;
   const int ix = a.ix, jx = a.jx;
   const size_t N = (size_t)ix * jx;
-  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * TY;
+  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * ty, nq = RX * (ty + 4);
   const bool perx = a.bc_kind[0] == OMHD_BC_PERIODIC, pery = a.bc_kind[2] == OMHD_BC_PERIODIC;
   const bool resist = a.eta_kind != OMHD_ETA_NONE;
   const double f1g = a.gm1;  // u2v.f90:11, derived on the host
@@ -207,16 +207,17 @@ __device__ __forceinline__ void phase_load(const StageArgs& a, int bxi, int byi,
   // converted, so their global-memory latencies overlap; FP32-mixed (two CTAs
   // per SM, 112 registers) one cell per pass
   constexpr int B = sizeof(T) == 8 ? 2 : 1;
-  for (int q0 = t; q0 < PL; q0 += B * n) {
+#pragma unroll 1
+  for (int q0 = t; q0 < nq; q0 += B * n) {
     double u[B][NV];
     bool act[B];
 #pragma unroll
     for (int b = 0; b < B; ++b) {
       const int q = q0 + b * n;
       const int rx = q % RX, ry = q / RX;
-      const bool cx_in = rx >= 2 && rx < TX + 2, cy_in = ry >= 2 && ry < TY + 2;
+      const bool cx_in = rx >= 2 && rx < TX + 2, cy_in = ry >= 2 && ry < ty + 2;
       // corners: only the diagonal neighbours are needed, by the resistive terms
-      act[b] = q < PL && (cx_in || cy_in || (resist && rx != 0 && rx != RX - 1 && ry != 0 && ry != RY - 1));
+      act[b] = q < nq && (cx_in || cy_in || (resist && rx != 0 && rx != RX - 1 && ry != 0 && ry != ty + 3));
       if (act[b]) {
         if constexpr (STAGED) {
           constexpr int SW = RX + 2;
@@ -235,7 +236,7 @@ __device__ __forceinline__ void phase_load(const StageArgs& a, int bxi, int byi,
       if (!act[b]) continue;
       const int q = q0 + b * n;
       const int rx = q % RX, ry = q / RX;
-      const bool cx_in = rx >= 2 && rx < TX + 2, cy_in = ry >= 2 && ry < TY + 2;
+      const bool cx_in = rx >= 2 && rx < TX + 2, cy_in = ry >= 2 && ry < ty + 2;
       const int gi = gi0 - 2 + rx, gj = gj0 - 2 + ry;
       double ps = u[b][PS];
       if (a.stage == 1) ps = glmf * ps;
@@ -257,12 +258,14 @@ __device__ __forceinline__ void phase_load(const StageArgs& a, int bxi, int byi,
 // phase B: slopes in x (cells rx = 1..TX+2 on tile rows) and y (rows
 // ry = 1..TY+2 on tile columns) -> face states of both directions
 template <class T, class G, int TAPE>
-__device__ __forceinline__ void phase_recon(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t, int n) {
-  constexpr int TX = G::TX, TY = G::TY, RX = G::RX, RY = G::RY, PL = RX * RY;
-  constexpr int NXS = G::NXS, NYS = G::NYS, XS = TX + 2;
+__device__ __forceinline__ void phase_recon(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t, int n,
+                                            const int ty = G::TY) {
+  constexpr int TX = G::TX, RX = G::RX, RY = G::RY, PL = RX * RY;
+  constexpr int NXS = G::NXS, NYS = G::NYS, XS = TX + 2;  // strides of the face-state planes
+  const int nxs = ty * XS, nys = (ty + 2) * TX;           // cells reconstructed in x and y
   const int ix = a.ix, jx = a.jx;
   const size_t N = (size_t)ix * jx;
-  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * TY;
+  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * ty;
   const bool perx = a.bc_kind[0] == OMHD_BC_PERIODIC, pery = a.bc_kind[2] == OMHD_BC_PERIODIC;
   const int lm = a.lm_type;
   const T* W = m.W;
@@ -270,14 +273,18 @@ __device__ __forceinline__ void phase_recon(const StageArgs& a, int bxi, int byi
     if (lm == LM_MINMOD || lm == LM_MC) {
       // two neighbouring cells per item: wm, w0, w1, w2 give the three slopes
       // of both cells (their shared difference once), 4 loads instead of 6;
-      // x pairs (cx, cx+1) of a row, y pairs (cy, cy+1) of a column
-      constexpr int XP = XS / 2, NXP = NXS / 2, NYP = NYS / 2;
-      static_assert(XS % 2 == 0 && (TY + 2) % 2 == 0, "cell pairs need even strip lengths");
+      // x pairs (cx, cx+1) of a row, y pairs (cy, cy+1) of a column; where ty is
+      // odd a column's last pair starts one cell early (its first cell is
+      // written twice, with the same values)
+      constexpr int XP = XS / 2;
+      static_assert(XS % 2 == 0, "cell pairs need an even row length");
+      const int NXP = nxs / 2, NYP = (ty + 3) / 2 * TX;
+#pragma unroll 1
       for (int p = t; p < NXP + NYP; p += n) {
         const bool xd = p < NXP;
         const int pp = xd ? p : p - NXP;
         // first cell of the pair: x (cx0, cy) / y (cx, cy0)
-        const int ca = xd ? 2 * (pp % XP) : pp % TX, cb = xd ? pp / XP : 2 * (pp / TX);
+        const int ca = xd ? 2 * (pp % XP) : pp % TX, cb = xd ? pp / XP : min(2 * (pp / TX), ty);
         const int o = xd ? (cb + 2) * RX + (ca + 1) : (cb + 1) * RX + (ca + 2);
         const int st = xd ? 1 : RX;
         const int i0 = xd ? cb * XS + ca : cb * TX + ca, di = xd ? 1 : TX;
@@ -291,7 +298,7 @@ __device__ __forceinline__ void phase_recon(const StageArgs& a, int bxi, int byi
           // global cells of the pair; the tile owns cx/cy = 1..TX/TY
           const int gi = xd ? gi0 - 1 + ca : gi0 + ca, gj = xd ? gj0 + cb : gj0 - 1 + cb;
           const int gi1 = xd ? gi + 1 : gi, gj1 = xd ? gj : gj + 1;
-          const int c0 = xd ? ca : cb, lim = xd ? TX : TY;
+          const int c0 = xd ? ca : cb, lim = xd ? TX : ty;
           own0 = c0 >= 1 && c0 <= lim && gi <= ix - 2 && gj <= jx - 2;
           own1 = c0 + 1 >= 1 && c0 + 1 <= lim && gi1 <= ix - 2 && gj1 <= jx - 2;
           tc0 = (size_t)tape_cell(gi, ix, perx) + (size_t)ix * tape_cell(gj, jx, pery);
@@ -320,11 +327,12 @@ __device__ __forceinline__ void phase_recon(const StageArgs& a, int bxi, int byi
       return;
     }
   }
-  for (int q = t; q < NXS + NYS; q += n) {
+#pragma unroll 1
+  for (int q = t; q < nxs + nys; q += n) {
     int o, st;
     T *dl, *dr;
     int qq;
-    if (q < NXS) {
+    if (q < nxs) {
       const int cx = q % XS, cy = q / XS;
       o = (cy + 2) * RX + (cx + 1);
       st = 1;
@@ -332,7 +340,7 @@ __device__ __forceinline__ void phase_recon(const StageArgs& a, int bxi, int byi
       dr = m.SRx;
       qq = q;
     } else {
-      qq = q - NXS;
+      qq = q - nxs;
       const int cx = qq % TX, cy = qq / TX;
       o = (cy + 1) * RX + (cx + 2);
       st = RX;
@@ -344,16 +352,16 @@ __device__ __forceinline__ void phase_recon(const StageArgs& a, int bxi, int byi
       for (int v = 0; v < NV; ++v) {
         T l, r;
         reconstruct_t<T, OMHD_FAST>(lm, W[v * PL + o - st], W[v * PL + o], W[v * PL + o + st], l, r);
-        dl[v * (q < NXS ? NXS : NYS) + qq] = l;
-        dr[v * (q < NXS ? NXS : NYS) + qq] = r;
+        dl[v * (q < nxs ? NXS : NYS) + qq] = l;
+        dr[v * (q < nxs ? NXS : NYS) + qq] = r;
       }
     } else {
       // this cell's global index; x cells cx = 0..TX+1 of row cy, y cells
       // cy = 0..TY+1 of column cx (the tile owns cx/cy = 1..TX/TY)
-      const bool xd = q < NXS;
+      const bool xd = q < nxs;
       const int cx = xd ? q % XS : qq % TX, cy = xd ? q / XS : qq / TX;
       const int gi = xd ? gi0 - 1 + cx : gi0 + cx, gj = xd ? gj0 + cy : gj0 - 1 + cy;
-      const bool own = (xd ? (cx >= 1 && cx <= TX) : (cy >= 1 && cy <= TY)) && gi <= ix - 2 && gj <= jx - 2;
+      const bool own = (xd ? (cx >= 1 && cx <= TX) : (cy >= 1 && cy <= ty)) && gi <= ix - 2 && gj <= jx - 2;
       const size_t tc = (TAPE == tape::kReplay || a.tlim)
                             ? (size_t)tape_cell(gi, ix, perx) + (size_t)ix * tape_cell(gj, jx, pery)
                             : 0;
@@ -375,25 +383,26 @@ __device__ __forceinline__ void phase_recon(const StageArgs& a, int bxi, int byi
 // non-periodic edge); uniform over the CTA, so the barrier that follows the
 // wall fixes is taken only by the tiles that have some
 template <class G>
-__device__ __forceinline__ bool tile_on_wall(const StageArgs& a, int bxi, int byi) {
-  const int gi0 = 1 + bxi * G::TX, gj0 = 1 + byi * G::TY;
+__device__ __forceinline__ bool tile_on_wall(const StageArgs& a, int bxi, int byi, const int ty = G::TY) {
+  const int gi0 = 1 + bxi * G::TX, gj0 = 1 + byi * ty;
   const int clx = (a.ix - 2) - gi0 + 1, cly = (a.jx - 2) - gj0 + 1;
   const bool wx = a.bc_kind[0] != OMHD_BC_PERIODIC && (gi0 == 1 || (clx >= 1 && clx <= G::TX));
-  const bool wy = a.bc_kind[2] != OMHD_BC_PERIODIC && (gj0 == 1 || (cly >= 1 && cly <= G::TY));
+  const bool wy = a.bc_kind[2] != OMHD_BC_PERIODIC && (gj0 == 1 || (cly >= 1 && cly <= ty));
   return wx || wy;
 }
 
 // wall face fixes after phase B: x walls (2D_reconnection/bc.f90:136-165),
 // y walls (2D_KH/bc.f90:55-83)
 template <class T, class G>
-__device__ __forceinline__ void phase_walls(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t, int n) {
-  constexpr int TX = G::TX, TY = G::TY, NXS = G::NXS, NYS = G::NYS, XS = TX + 2;
+__device__ __forceinline__ void phase_walls(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t, int n,
+                                            const int ty = G::TY) {
+  constexpr int TX = G::TX, NXS = G::NXS, NYS = G::NYS, XS = TX + 2;
   const int ix = a.ix, jx = a.jx;
-  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * TY;
+  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * ty;
   if (a.bc_kind[0] != OMHD_BC_PERIODIC) {
     const int cl = (ix - 2) - gi0 + 1;  // cx of the last interior cell
-    for (int k = t; k < TY * NV; k += n) {
-      const int cy = k % TY, v = k / TY;
+    for (int k = t; k < ty * NV; k += n) {
+      const int cy = k % ty, v = k / ty;
       if (gi0 == 1) {  // west face: VL = flip(VR)
         const T s = m.SRx[v * NXS + cy * XS + 1];
         m.SLx[v * NXS + cy * XS + 0] = ((a.bc_flip[0] >> v) & 1) ? -s : s;
@@ -413,7 +422,7 @@ __device__ __forceinline__ void phase_walls(const StageArgs& a, int bxi, int byi
         const T s = m.SRy[v * NYS + 1 * TX + cx];
         m.SLy[v * NYS + 0 * TX + cx] = ((a.bc_flip[2] >> v) & 1) ? -s : s;
       }
-      if (cl >= 1 && cl <= TY) {  // north face: VR = flip(VL)
+      if (cl >= 1 && cl <= ty) {  // north face: VR = flip(VL)
         const T s = m.SLy[v * NYS + cl * TX + cx];
         m.SRy[v * NYS + (cl + 1) * TX + cx] = ((a.bc_flip[3] >> v) & 1) ? -s : s;
       }
@@ -436,19 +445,21 @@ __device__ __forceinline__ constexpr int rot_y(int k) {
 // direction to whole warps: 18).
 template <class T, int FLUX, class G, int TAPE>
 __device__ __forceinline__ void phase_flux_rot(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t,
-                                               int n, const StageScalars<T>& ks) {
+                                               int n, const StageScalars<T>& ks, const int ty) {
   constexpr int TX = G::TX, RX = G::RX;
-  constexpr int NXS = G::NXS, NYS = G::NYS, NXF = G::NXF, NYF = G::NYF, XS = TX + 2, XF = TX + 1;
+  constexpr int NXS = G::NXS, NYS = G::NYS, XS = TX + 2, XF = TX + 1;
+  const int nxf = ty * XF, nyf = (ty + 1) * TX;  // x and y faces
   constexpr int PL = RX * G::RY;
   const int ix = a.ix, jx = a.jx;
   const size_t N = (size_t)ix * jx;
-  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * G::TY;
+  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * ty;
   const bool resist = a.eta_kind != OMHD_ETA_NONE;
   const T ch = ks.ch, gam = ks.gam, r1 = ks.r1, r2 = ks.r2;
   const T* W = m.W;
-  for (int q = t; q < NXF + NYF; q += n) {
-    const bool xd = q < NXF;
-    const int qq = xd ? q : q - NXF;
+#pragma unroll 1
+  for (int q = t; q < nxf + nyf; q += n) {
+    const bool xd = q < nxf;
+    const int qq = xd ? q : q - nxf;
     // x face (fx, cy): lower cell fx of x row cy; y face (cx, fy): lower cell
     // fy of y column cx
     const int fa = xd ? qq % XF : qq % TX, fb = xd ? qq / XF : qq / TX;
@@ -526,9 +537,9 @@ __device__ __forceinline__ void phase_flux_rot(const StageArgs& a, int bxi, int 
 // warps) and all y faces (items NXFP..NXFP+NYF-1)
 template <class T, int FLUX, class G, int TAPE>
 __device__ __forceinline__ void phase_flux(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t, int n,
-                                           const StageScalars<T>& ks) {
+                                           const StageScalars<T>& ks, const int ty = G::TY) {
   if constexpr (OMHD_FAST && sizeof(T) == 8) {
-    phase_flux_rot<T, FLUX, G, TAPE>(a, bxi, byi, m, t, n, ks);
+    phase_flux_rot<T, FLUX, G, TAPE>(a, bxi, byi, m, t, n, ks, ty);
     return;
   }
   constexpr int TX = G::TX, RX = G::RX;
@@ -541,6 +552,7 @@ __device__ __forceinline__ void phase_flux(const StageArgs& a, int bxi, int byi,
   const T ch = ks.ch, gam = ks.gam, r1 = ks.r1, r2 = ks.r2;
   const T* W = m.W;
   constexpr int XF = TX + 1;
+#pragma unroll 1
   for (int q = t; q < NXFP + NYF; q += n) {
     if (q < NXFP) {
       if (q >= NXF) continue;  // padding lanes
@@ -623,11 +635,11 @@ __device__ __forceinline__ void phase_flux(const StageArgs& a, int bxi, int byi,
 // grid's maximum, given that it is known or more; or 0
 template <class T, class G>
 __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t,
-                                               int n, const StageScalars<T>& ks, float known) {
-  constexpr int TX = G::TX, TY = G::TY;
+                                               int n, const StageScalars<T>& ks, float known, const int rows = G::TY) {
+  constexpr int TX = G::TX;
   const int ix = a.ix, jx = a.jx;
   const size_t N = (size_t)ix * jx;
-  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * TY;
+  const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * rows;
   const bool perx = a.bc_kind[0] == OMHD_BC_PERIODIC, pery = a.bc_kind[2] == OMHD_BC_PERIODIC;
   const double gamma = a.gamma;
   const double f1g = a.gm1;
@@ -645,7 +657,8 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
 #pragma unroll
   for (int q = 0; q < 4; ++q) flip[q] = a.bc_flip[q];
   double vcell = 0.0;
-  for (int k = t; k < TX * TY; k += n) {
+#pragma unroll 1
+  for (int k = t; k < TX * rows; k += n) {
     const int tx = k % TX, ty = k / TX;
     const int gi = gi0 + tx, gj = gj0 + ty;
     if (gi > ix - 2 || gj > jx - 2) continue;
@@ -773,16 +786,22 @@ __global__ void __launch_bounds__(GeoFor<T>::type::NT, sizeof(T) == 4 ? OMHD_MIX
 
 // ---------------------------------------------------------------------------
 // FP64 pipelined stage kernel: one persistent CTA per SM, warp-specialised.
-// The flux phase C is FP64-pipe bound (~96 % of the pipe), while the load +
-// u2v phase A, the slope phase B and the update phase D are latency bound
-// (~50 %).  So NPW producer warps run A and B (+ wall fixes) of tile i+1
-// while the 9 consumer warps run C and D of tile i: two face-state buffers in
+// The phases differ in how much of the FP64 pipe they can use (a warp has one
+// FP64 operation in flight, 64 cycles; the pipe takes one in 19), so NPW producer
+// warps run A and B (+ wall fixes) of tile i+1 while the 9 consumer warps run C
+// and D of tile i: two face-state buffers in
 // shared memory, handed over with named barriers (FULL[b]: producers arrive,
 // consumers wait; EMPTY[b]: consumers arrive after D, producers wait before
 // refilling b).  Fluxes overwrite the lower-cell face state that only their
 // own face reads, so a buffer is 4 face-state arrays (83 KB) and the CTA holds
-// W + 2 buffers = 195 KB.  Non-resistive 2D runs (the resistive terms read W
-// in phase C, which the producers already refill).
+// W + 2 buffers = 195 KB.  Tiles are 16 cells wide and ty <= 16 rows high
+// (pick_rows); the loops over a tile run to ty, which also keeps them rolled: the
+// unrolled flux loop (two copies of the solver) cost 8 % in instruction fetches.
+// Non-resistive 2D runs (the resistive terms read W in phase C, which the
+// producers already refill).
+// Measured on KH 4096x2048, ms per step: 20.3 with the FP64-pipe arithmetic, 17.7
+// with integer reciprocals and roots, 14.1 with integer products, 12.9 rolled and
+// with the CFL bound; FP64 pipe 76 % busy (84 % is all it gives with 12 warps).
 // ---------------------------------------------------------------------------
 using PipeGeo = Geo2<16, 16>;
 constexpr int kPipeBarProd = 1, kPipeBarCons = 2, kPipeBarFull = 3, kPipeBarEmpty = 5;
@@ -828,7 +847,7 @@ __device__ __forceinline__ TileMem<double> pipe_mem(unsigned char* smem_raw, int
 
 template <int FLUX, int TAPE, int NPW>
 __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
-    k_stage2d_pipe(const StageArgs a, const __grid_constant__ CUtensorMap tmap, const int use_tma) {
+    k_stage2d_pipe(const StageArgs a, const __grid_constant__ CUtensorMap tmap, const int use_tma, const int ty) {
   using G = PipeGeo;
   constexpr int NP = NPW * 32, NC = G::NT, NTOT = NP + NC;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -845,58 +864,70 @@ __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
   if (skip) return;
   const double glmf = ks.glmf;
   const int ntx = (a.ix - 2 + G::TX - 1) / G::TX;
-  const int ntiles = ntx * ((a.jx - 2 + G::TY - 1) / G::TY);
+  const int ntiles = ntx * ((a.jx - 2 + ty - 1) / ty);
   double vmax = 0.0;
-  if (threadIdx.x < NP) {  // producers: A, B, wall fixes of tiles blockIdx.x, +gridDim.x, ...
+  // TMA staging: a tile whose whole halo lies inside the array (no periodic
+  // wrap, no wall clamp, no ragged edge) arrives as one 3D box load issued
+  // by producer thread 0 while the producers work on the previous tile; the
+  // other tiles take ordinary loads.  The box starts one cell left of the
+  // halo so that its x coordinate is even (8-byte elements, 16-byte rule).
+  unsigned char* s0 = smem_raw + pipe_stage_off();
+  double* S = reinterpret_cast<double*>(s0 + ((128u - (smem_u32(s0) & 127u)) & 127u));  // 128-byte aligned
+  auto staged = [&](int w) {
+    if (!use_tma) return false;
+    const int gi0 = 1 + (w % ntx) * G::TX, gj0 = 1 + (w / ntx) * ty;
+    return gi0 >= 3 && gj0 >= 2 && gi0 - 2 + G::RX <= a.ix && gj0 - 2 + G::RY <= a.jx;
+  };
+  auto issue = [&](int w) {
+    const int gi0 = 1 + (w % ntx) * G::TX, gj0 = 1 + (w / ntx) * ty;
+    fence_proxy_async_smem();  // the producers' reads of S come before this write
+    mbar_arrive_expect_tx(&tma_bar, kPipeBoxBytes);
+    tma_load_3d(S, &tmap, gi0 - 3, gj0 - 2, 0, &tma_bar);
+  };
+  // A and B of the CTA's first tile by all its warps: with the producers alone
+  // the others would wait for it, which on a small grid (one tile per CTA) is
+  // a third of the launch
+  const int wfirst = blockIdx.x, wsecond = wfirst + (int)gridDim.x;
+  {
+    if (use_tma && threadIdx.x == 0) mbar_init(&tma_bar, 1);
+    const TileMem<double> m = pipe_mem(smem_raw, 0);
+    phase_load<double, G>(a, wfirst % ntx, wfirst / ntx, m, threadIdx.x, NTOT, glmf, nullptr, ty);
+    __syncthreads();
+    if (threadIdx.x == 0 && wsecond < ntiles && staged(wsecond)) issue(wsecond);
+    phase_recon<double, G, TAPE>(a, wfirst % ntx, wfirst / ntx, m, threadIdx.x, NTOT, ty);
+    __syncthreads();
+    if (tile_on_wall<G>(a, wfirst % ntx, wfirst / ntx, ty)) {
+      phase_walls<double, G>(a, wfirst % ntx, wfirst / ntx, m, threadIdx.x, NTOT, ty);
+      __syncthreads();
+    }
+  }
+  if (threadIdx.x < NP) {  // producers: A, B, wall fixes of the CTA's further tiles
     const int t = threadIdx.x;
-    // TMA staging: a tile whose whole halo lies inside the array (no periodic
-    // wrap, no wall clamp, no ragged edge) arrives as one 3D box load issued
-    // by producer thread 0 while the producers work on the previous tile; the
-    // other tiles take ordinary loads.  The box starts one cell left of the
-    // halo so that its x coordinate is even (8-byte elements, 16-byte rule).
-    unsigned char* s0 = smem_raw + pipe_stage_off();
-    double* S = reinterpret_cast<double*>(s0 + ((128u - (smem_u32(s0) & 127u)) & 127u));  // 128-byte aligned
-    auto staged = [&](int w) {
-      if (!use_tma) return false;
-      const int gi0 = 1 + (w % ntx) * G::TX, gj0 = 1 + (w / ntx) * G::TY;
-      return gi0 >= 3 && gj0 >= 2 && gi0 - 2 + G::RX <= a.ix && gj0 - 2 + G::RY <= a.jx;
-    };
-    auto issue = [&](int w) {
-      const int gi0 = 1 + (w % ntx) * G::TX, gj0 = 1 + (w / ntx) * G::TY;
-      fence_proxy_async_smem();  // the producers' reads of S come before this write
-      mbar_arrive_expect_tx(&tma_bar, kPipeBoxBytes);
-      tma_load_3d(S, &tmap, gi0 - 3, gj0 - 2, 0, &tma_bar);
-    };
     uint32_t tphase = 0;
     bool tma_lost = false;
-    if (use_tma) {
-      if (t == 0) mbar_init(&tma_bar, 1);
-      named_bar_sync(kPipeBarProd, NP);
-      if (t == 0 && (int)blockIdx.x < ntiles && staged(blockIdx.x)) issue(blockIdx.x);
-    }
-    int i = 0;
-    for (int w = blockIdx.x; w < ntiles; w += gridDim.x, ++i) {
+    int i = 1;
+    for (int w = wsecond; w < ntiles; w += gridDim.x, ++i) {
       const int b = i & 1;
       const TileMem<double> m = pipe_mem(smem_raw, b);
       if (i >= 2) named_bar_sync(kPipeBarEmpty + b, NTOT);  // consumers are done with buffer b
-      if (i >= 1) named_bar_sync(kPipeBarProd, NP);         // W of the previous tile is read
+      if (i >= 2) named_bar_sync(kPipeBarProd, NP);         // W of the previous tile is read
       if (staged(w) && !tma_lost) {
         if (!mbar_wait_parity(&tma_bar, tphase & 1u, kTmaMaxPolls)) {
           tma_lost = true;  // recorded; the tile's results are void, the protocol goes on
-          raise_error(a.err, OMHD_TIMEOUT, 1 + (w % ntx) * G::TX, 1 + (w / ntx) * G::TY, 0, 0, 0.0);
+          raise_error(a.err, OMHD_TIMEOUT, 1 + (w % ntx) * G::TX, 1 + (w / ntx) * ty, 0, 0, 0.0);
         }
         ++tphase;
-        phase_load<double, G, true>(a, w % ntx, w / ntx, m, t, NP, glmf, S);
+        phase_load<double, G, true>(a, w % ntx, w / ntx, m, t, NP, glmf, S, ty);
       } else {
-        phase_load<double, G>(a, w % ntx, w / ntx, m, t, NP, glmf);
+        phase_load<double, G>(a, w % ntx, w / ntx, m, t, NP, glmf, nullptr, ty);
       }
       named_bar_sync(kPipeBarProd, NP);
       const int wn = w + (int)gridDim.x;
       if (t == 0 && !tma_lost && wn < ntiles && staged(wn)) issue(wn);
-      phase_recon<double, G, TAPE>(a, w % ntx, w / ntx, m, t, NP);
-      if (tile_on_wall<G>(a, w % ntx, w / ntx)) {
+      phase_recon<double, G, TAPE>(a, w % ntx, w / ntx, m, t, NP, ty);
+      if (tile_on_wall<G>(a, w % ntx, w / ntx, ty)) {
         named_bar_sync(kPipeBarProd, NP);
-        phase_walls<double, G>(a, w % ntx, w / ntx, m, t, NP);
+        phase_walls<double, G>(a, w % ntx, w / ntx, m, t, NP, ty);
       }
       __threadfence_block();
       named_bar_arrive(kPipeBarFull + b, NTOT);
@@ -909,11 +940,11 @@ __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
     for (int w = blockIdx.x; w < ntiles; w += gridDim.x, ++i) {
       const int b = i & 1;
       const TileMem<double> m = pipe_mem(smem_raw, b);
-      named_bar_sync(kPipeBarFull + b, NTOT);
+      if (i >= 1) named_bar_sync(kPipeBarFull + b, NTOT);
       const float known = a.stage == 2 ? cfl_known(st) : 0.0f;
-      phase_flux<double, FLUX, G, TAPE>(a, w % ntx, w / ntx, m, t, NC, ks);
+      phase_flux<double, FLUX, G, TAPE>(a, w % ntx, w / ntx, m, t, NC, ks, ty);
       named_bar_sync(kPipeBarCons, NC);
-      const double v = phase_update<double, G>(a, w % ntx, w / ntx, m, t, NC, ks, known);
+      const double v = phase_update<double, G>(a, w % ntx, w / ntx, m, t, NC, ks, known, ty);
       if (a.stage == 2) cfl_publish(st, v, known);
       vmax = lt_<double, OMHD_FAST>(vmax, v) ? v : vmax;
       if (i + 2 < nmine) {  // the producers refill buffer b for tile i+2
@@ -933,6 +964,28 @@ __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
 #ifndef OMHD_PIPE_PRODUCER_WARPS
 #define OMHD_PIPE_PRODUCER_WARPS 3
 #endif
+// Rows per tile of the pipelined kernel for a grid of ntx tile columns and ny
+// rows on nsm SMs.  Measured on GB300 over 64^2 .. 700^2 grids and 3 .. 16 rows, a
+// step takes rounds x (16 + 3.4 rows) + 31 us, rounds = the tiles of the busiest
+// SM: the split with the smallest rounds x (rows + 4.7) is taken.  Small grids get
+// low tiles on all SMs (64^2: 115 us a step with 16 rows, 60 with 4), middle-sized
+// ones a count that fills the last round (256^2: 172 us with 16 rows, two tiles on
+// 104 of 152 SMs; 164 with 14, two on every SM), large ones 16 rows, whose halo
+// is the smallest.  Below 4 rows nothing is gained.
+inline int pick_rows(int ntx, int ny, int nsm) {
+  int best = PipeGeo::TY;
+  double best_cost = 1e300;
+  for (int ty = PipeGeo::TY; ty >= 4; --ty) {
+    const long long tiles = (long long)ntx * ((ny + ty - 1) / ty);
+    const double cost = (double)((tiles + nsm - 1) / nsm) * (ty + 4.7);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = ty;
+    }
+  }
+  return best;
+}
+
 template <int FLUX, int TAPE, int NPW = OMHD_PIPE_PRODUCER_WARPS>
 int launch_pipe(const StageArgs& a, cudaStream_t s) {
   const size_t bytes = pipe_smem_bytes_tma();
@@ -943,7 +996,9 @@ int launch_pipe(const StageArgs& a, cudaStream_t s) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return (int)e;
-  const int ntiles = ((a.ix - 2 + PipeGeo::TX - 1) / PipeGeo::TX) * ((a.jx - 2 + PipeGeo::TY - 1) / PipeGeo::TY);
+  const int ntx = (a.ix - 2 + PipeGeo::TX - 1) / PipeGeo::TX;
+  const int ty = pick_rows(ntx, a.jx - 2, nsm);
+  const int ntiles = ntx * ((a.jx - 2 + ty - 1) / ty);
   const int grid = ntiles < nsm ? ntiles : nsm;
   // the tensor map of this stage's input state (encoded on the host, passed by
   // value; an array TMA cannot address -- odd ix, unaligned base -- is loaded
@@ -952,7 +1007,7 @@ int launch_pipe(const StageArgs& a, cudaStream_t s) {
   memset(&tmap, 0, sizeof tmap);
   const int use_tma =
       tma_staging_enabled() && tma_encode_state_map(&tmap, a.Uin, a.ix, a.jx, NV, kPipeBoxX, kPipeBoxY) == 0;
-  k_stage2d_pipe<FLUX, TAPE, NPW><<<grid, NPW * 32 + PipeGeo::NT, bytes, s>>>(a, tmap, use_tma);
+  k_stage2d_pipe<FLUX, TAPE, NPW><<<grid, NPW * 32 + PipeGeo::NT, bytes, s>>>(a, tmap, use_tma, ty);
   return (int)cudaGetLastError();
 }
 
