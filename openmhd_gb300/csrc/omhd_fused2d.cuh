@@ -664,34 +664,47 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
     if (gi > ix - 2 || gj > jx - 2) continue;
     const size_t c = (size_t)gi + (size_t)ix * gj;
     double out[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      // F(i-1/2) - F(i+1/2) in FP64
+    // The alternatives (grid spacing, RK stage) are chosen outside the loops over
+    // the variables, in blocks too long to be predicated: a predicated-off FP64
+    // instruction holds the FP64 pipe like any other, and with the choices inside
+    // the ensemble kernel spent half of its FP64 time on the results not taken.
+    auto dF = [&](int v) {  // F(i-1/2) - F(i+1/2) in FP64
       const double* fx = m.FX + v * m.fxv + ty * m.fxr + tx;
-      const double dF = fx[0] - fx[1];
-      const double gm = m.FY[v * m.fyv + ty * TX + tx], gp = m.FY[v * m.fyv + (ty + 1) * TX + tx];
-      if constexpr (OMHD_FAST && sizeof(T) == 8) {
-        // rk.f90:26-35, :56-66 as U + dt/dx (dF + dx/dy dG): 4 (stage 1) or 5 FP64
-        // operations a variable instead of 5 or 8, as many roundings of the sum
-        const double ub = v == PS ? glmf * Ubase[v * N + c] : Ubase[v * N + c];
-        const double d = fma(ryx, gm - gp, dF);
-        if (rk2)
-          out[v] = fma(dtx, d, ub);
-        else
-          out[v] = half_exact(fma(dtx, d, ub + U1[v * N + c]));
-        continue;
+      return fx[0] - fx[1];
+    };
+    auto gm = [&](int v) { return m.FY[v * m.fyv + ty * TX + tx]; };
+    auto gp = [&](int v) { return m.FY[v * m.fyv + (ty + 1) * TX + tx]; };
+    double u0[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) u0[v] = Ubase[v * N + c];
+    auto ub = [&](int v) { return v == PS ? glmf * u0[v] : u0[v]; };
+    if constexpr (OMHD_FAST && sizeof(T) == 8) {
+      // rk.f90:26-35, :56-66 as U + dt/dx (dF + dx/dy dG): 4 (stage 1) or 5 FP64
+      // operations a variable instead of 5 or 8, as many roundings of the sum
+      if (rk2) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) out[v] = fma(dtx, fma(ryx, gm(v) - gp(v), dF(v)), ub(v));
+      } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+          out[v] = half_exact(fma(dtx, fma(ryx, gm(v) - gp(v), dF(v)), ub(v) + U1[v * N + c]));
       }
-      double d;
-      if (iso)
-        d = dtx * (dF + gm - gp);  // rk.f90:26-35 operation order
-      else
-        d = dtx * dF + dty * (gm - gp);
-      double ub = Ubase[v * N + c];
-      if (v == PS) ub = glmf * ub;
-      if (rk2)
-        out[v] = ub + d;  // rk_tvd21 / rk_std21 / rk_std22
-      else
-        out[v] = 0.5 * (ub + U1[v * N + c] + d);  // rk_tvd22 (rk.f90:56-66)
+    } else {
+      double d[NV];
+      if (iso) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) d[v] = dtx * (dF(v) + gm(v) - gp(v));  // rk.f90:26-35 operation order
+      } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) d[v] = dtx * dF(v) + dty * (gm(v) - gp(v));
+      }
+      if (rk2) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) out[v] = ub(v) + d[v];  // rk_tvd21 / rk_std21 / rk_std22
+      } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) out[v] = 0.5 * (ub(v) + U1[v * N + c] + d[v]);  // rk_tvd22 (rk.f90:56-66)
+      }
     }
     if (stage2) out[PS] = glmf * out[PS];  // second GLM half (main.f90:185)
 

@@ -548,27 +548,36 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
     if (own && !lead) {
       const size_t c = (size_t)gi + (size_t)ix * ((size_t)gj + (size_t)jx * k);
       double out[NV];
+      // the alternatives outside the loops over the variables: predicated-off FP64
+      // instructions hold the FP64 pipe (164 of its instructions a cell and stage
+      // in the mixed kernel for 89 operations, with the choices inside)
+      const bool rk2 = a.stage == 1 || a.time_type == OMHD_TIME_RK2;
+      auto ub = [&](int v) { return v == PS ? glmf * a.Ubase[v * N + c] : a.Ubase[v * N + c]; };
+      if constexpr (OMHD_FAST && sizeof(T) == 8) {  // U + dt/dx (dF + dx/dy dG + dx/dz dH)
+        auto d = [&](int v) { return fma(a.rzx, Fzp[v] - Fzc[v], fma(a.ryx, gm[v] - gp[v], acc[v])); };
+        if (rk2) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        if constexpr (OMHD_FAST && sizeof(T) == 8) {  // U + dt/dx (dF + dx/dy dG + dx/dz dH)
-          const double ub = v == PS ? glmf * a.Ubase[v * N + c] : a.Ubase[v * N + c];
-          const bool rk2 = a.stage == 1 || a.time_type == OMHD_TIME_RK2;
-          const double u0 = rk2 ? ub : ub + a.U1[v * N + c];
-          const double d = fma(dtx, fma(a.rzx, Fzp[v] - Fzc[v], fma(a.ryx, gm[v] - gp[v], acc[v])), u0);
-          out[v] = rk2 ? d : half_exact(d);
-          continue;
+          for (int v = 0; v < NV; ++v) out[v] = fma(dtx, d(v), ub(v));
+        } else {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) out[v] = half_exact(fma(dtx, d(v), ub(v) + a.U1[v * N + c]));
         }
-        double d;
-        if (a.iso)
-          d = dtx * (acc[v] + gm[v] - gp[v] + Fzp[v] - Fzc[v]);  // 3D_basic/rk.f90:26-35 order
-        else
-          d = dtx * acc[v] + dty * (gm[v] - gp[v]) + dtz * (Fzp[v] - Fzc[v]);
-        double ub = a.Ubase[v * N + c];
-        if (v == PS) ub = glmf * ub;
-        if (a.stage == 1 || a.time_type == OMHD_TIME_RK2)
-          out[v] = ub + d;
-        else
-          out[v] = 0.5 * (ub + a.U1[v * N + c] + d);
+      } else {
+        double d[NV];
+        if (a.iso) {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) d[v] = dtx * (acc[v] + gm[v] - gp[v] + Fzp[v] - Fzc[v]);  // 3D_basic/rk.f90:26-35 order
+        } else {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) d[v] = dtx * acc[v] + dty * (gm[v] - gp[v]) + dtz * (Fzp[v] - Fzc[v]);
+        }
+        if (rk2) {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) out[v] = ub(v) + d[v];
+        } else {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) out[v] = 0.5 * (ub(v) + a.U1[v * N + c] + d[v]);
+        }
       }
       if (a.stage == 2) out[PS] = glmf * out[PS];
       int xt[3], yt[3], zt[3], xf[3], yf[3], zf[3], nxt = 1, nyt = 1, nzt = 1;
