@@ -25,7 +25,26 @@ namespace omhd {
 namespace OMHD_VARIANT {
 namespace d3 {
 
-// column of the one-role kernel (build-time constants, for tuning)
+// A column of TX x TY cells and the CTAs per SM its kernel is built for.
+template <int TX_, int TY_, int CTAS_>
+struct Col {
+  static constexpr int TX = TX_, TY = TY_, CTAS = CTAS_, NT = TX * TY;
+  static_assert(TY * NV <= NT - TX, "the x and y wall fixes use disjoint threads");
+  static constexpr int RX = TX + 4, RY = TY + 4, PL = RX * RY;  // plane of the halo tile
+  static constexpr int XS = TX + 2, NXS3 = TY * XS;             // cells reconstructed in x (a row strip per tile row)
+  static constexpr int NYS3 = (TY + 2) * TX;                    // cells reconstructed in y
+  static constexpr int XF = TX + 1, NXF3 = TY * XF;             // x faces
+  static constexpr int NXFP3 = (NXF3 + 31) / 32 * 32;           // x faces padded to whole warps
+  static constexpr int NYF3 = (TY + 1) * TX;                    // y faces
+  // ring of NRING primitive planes, then the x and y face states of one plane;
+  // each face's flux overwrites the lower-cell face state that only it reads
+  template <class T>
+  static constexpr size_t smem_bytes() {
+    return sizeof(T) * (size_t)NV * (4 * PL + 2 * NXS3 + 2 * NYS3);
+  }
+};
+// The column of the other builds than the FP64 performance one: 32x8, FP32 two
+// CTAs per SM (build-time constants, for tuning)
 #ifndef OMHD_3D_TILE_X
 #define OMHD_3D_TILE_X 32
 #endif
@@ -35,15 +54,12 @@ namespace d3 {
 #ifndef OMHD_3D_MIXED_MIN_CTAS  // resident CTAs per SM the FP32-mixed 3D kernel is built for
 #define OMHD_3D_MIXED_MIN_CTAS 2
 #endif
-constexpr int TX = OMHD_3D_TILE_X, TY = OMHD_3D_TILE_Y, NT = TX * TY;
-static_assert(TY * NV <= NT - TX, "the x and y wall fixes use disjoint threads");
-constexpr int RX = TX + 4, RY = TY + 4, PL = RX * RY;  // plane of the halo tile
+template <class T>
+using DefaultCol = Col<OMHD_3D_TILE_X, OMHD_3D_TILE_Y, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 1>;
+// FP64 HLLD with fused multiply-adds: 16x16, or two 16x8 CTAs per SM (pick_col)
+using WideCol = Col<16, 16, 1>;
+using SmallCol = Col<16, 8, 2>;
 constexpr int NRING = 4;
-constexpr int XS = TX + 2, NXS3 = TY * XS;        // cells reconstructed in x (a row strip per tile row)
-constexpr int NYS3 = (TY + 2) * TX;               // cells reconstructed in y
-constexpr int XF = TX + 1, NXF3 = TY * XF;        // x faces
-constexpr int NXFP3 = (NXF3 + 31) / 32 * 32;      // x faces padded to whole warps
-constexpr int NYF3 = (TY + 1) * TX;               // y faces
 constexpr int ZCHUNK = 64;  // most z planes marched by one CTA
 
 // z planes per CTA for a grid of `columns` columns and nz interior planes on a
@@ -56,7 +72,7 @@ constexpr int ZCHUNK = 64;  // most z planes marched by one CTA
 // 12.3 -> 0.95 (8 CTAs before), field loop 100x100x200 FP64 15.9 -> 10.4 (208 CTAs
 // in two rounds), Harris 256x128x256 mixed 10.5 -> 9.4 (512 CTAs on 304 slots).
 constexpr double kProloguePlanes = 1.5;
-inline int pick_zchunk(long long columns, int nz, int slots) {
+inline int pick_zchunk(long long columns, int nz, int slots, double* cost_out = nullptr) {
   int best = ZCHUNK;
   double best_cost = 1e300;
   for (int c = nz < ZCHUNK ? nz : ZCHUNK; c >= 1; --c) {
@@ -68,14 +84,8 @@ inline int pick_zchunk(long long columns, int nz, int slots) {
       best = c;
     }
   }
+  if (cost_out) *cost_out = best_cost;
   return best;
-}
-
-// ring of NRING primitive planes, then the x and y face states of one plane;
-// each face's flux overwrites the lower-cell face state that only it reads
-template <class T>
-constexpr size_t smem3d_bytes() {
-  return sizeof(T) * (size_t)NV * (NRING * PL + 2 * NXS3 + 2 * NYS3);
 }
 
 __device__ __forceinline__ int map_idx(int g, int n, bool periodic) {
@@ -145,11 +155,49 @@ __device__ __forceinline__ void resist_face_f32(const BF& b, float eta_dx, float
   }
 }
 
+// The same terms of the FP64 kernels, added to the face flux F (grid components);
+// b as above, n = 0, 1, 2 the face normal's axis.
+template <int n, class BF>
+__device__ __forceinline__ void resist_face_f64(const BF& B, double eta_dx, double (&F)[NV]) {
+  if constexpr (n == 0) {  // flux_resistive.cuf:87-101
+    const double JyS = -(B(BZ, 1, 0, 0) - B(BZ, 0, 0, 0)) +
+                       0.25 * (B(BX, 0, 0, 1) + B(BX, 1, 0, 1) - B(BX, 0, 0, -1) - B(BX, 1, 0, -1));
+    const double JzS = (B(BY, 1, 0, 0) - B(BY, 0, 0, 0)) -
+                       0.25 * (B(BX, 0, 1, 0) + B(BX, 1, 1, 0) - B(BX, 0, -1, 0) - B(BX, 1, -1, 0));
+    F[EN] = F[EN] + 0.5 * eta_dx * (JyS * (B(BZ, 0, 0, 0) + B(BZ, 1, 0, 0)) - JzS * (B(BY, 0, 0, 0) + B(BY, 1, 0, 0)));
+    F[BY] = F[BY] - eta_dx * JzS;
+    F[BZ] = F[BZ] + eta_dx * JyS;
+  } else if constexpr (n == 1) {  // flux_resistive.cuf:104-118
+    const double JxS = (B(BZ, 0, 1, 0) - B(BZ, 0, 0, 0)) -
+                       0.25 * (B(BY, 0, 0, 1) + B(BY, 0, 1, 1) - B(BY, 0, 0, -1) - B(BY, 0, 1, -1));
+    const double JzS = -(B(BX, 0, 1, 0) - B(BX, 0, 0, 0)) +
+                       0.25 * (B(BY, 1, 0, 0) + B(BY, 1, 1, 0) - B(BY, -1, 0, 0) - B(BY, -1, 1, 0));
+    F[EN] = F[EN] + 0.5 * eta_dx * (JzS * (B(BX, 0, 0, 0) + B(BX, 0, 1, 0)) - JxS * (B(BZ, 0, 0, 0) + B(BZ, 0, 1, 0)));
+    F[BX] = F[BX] + eta_dx * JzS;
+    F[BZ] = F[BZ] - eta_dx * JxS;
+  } else {  // flux_resistive.cuf:121-135
+    const double JyS = (B(BX, 0, 0, 1) - B(BX, 0, 0, 0)) -
+                       0.25 * (B(BZ, 1, 0, 0) + B(BZ, 1, 0, 1) - B(BZ, -1, 0, 0) - B(BZ, -1, 0, 1));
+    const double JxS = -(B(BY, 0, 0, 1) - B(BY, 0, 0, 0)) +
+                       0.25 * (B(BZ, 0, 1, 0) + B(BZ, 0, 1, 1) - B(BZ, 0, -1, 0) - B(BZ, 0, -1, 1));
+    F[EN] = F[EN] + 0.5 * eta_dx * (JxS * (B(BY, 0, 0, 0) + B(BY, 0, 0, 1)) - JyS * (B(BX, 0, 0, 0) + B(BX, 0, 0, 1)));
+    F[BX] = F[BX] - eta_dx * JyS;
+    F[BY] = F[BY] + eta_dx * JxS;
+  }
+}
+
+// slot k of a face state rotated into x orientation holds component rot3(n, k) for
+// the face normal n = 0, 1, 2 (x, y, z), the component order of flux_solver.f90
+__device__ __forceinline__ constexpr int rot3(int n, int k) {
+  return (k <= 2) ? (k + n) % 3 : ((k >= 5 && k <= 7) ? 5 + (k - 5 + n) % 3 : k);
+}
+
 // Load + convert one z plane (global index gk, any value; mapped by the z bc)
 // of the halo tile into ring slot `slot`.
-template <class T>
+template <class T, class G>
 __device__ __forceinline__ void load_plane(const StageArgs& a, T* W, int slot, int gk, int gi0, int gj0, bool perx,
                                            bool pery, bool perz, bool resist, double glmf, bool own_plane) {
+  constexpr int TX = G::TX, TY = G::TY, NT = G::NT, RX = G::RX, RY = G::RY, PL = G::PL;
   const int ix = a.ix, jx = a.jx, kx = a.kx;
   const size_t N = (size_t)ix * jx * kx;
   const double f1g = a.gm1;  // derived on the host
@@ -187,9 +235,10 @@ __device__ __forceinline__ void load_plane(const StageArgs& a, T* W, int slot, i
 // FP32 face arithmetic: two CTAs per SM (registers capped at 128, 97 KB of
 // shared memory each), so that one CTA's FP64 loads, updates and barriers
 // overlap the other's face work.
-template <class T, int FLUX>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 1)
-    k_stage3d(const StageArgs a, const int zchunk) {
+template <class T, int FLUX, class G>
+__global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, const int zchunk) {
+  constexpr int TX = G::TX, TY = G::TY, NT = G::NT, RX = G::RX, PL = G::PL, XS = G::XS, XF = G::XF;
+  constexpr int NXS3 = G::NXS3, NYS3 = G::NYS3, NXF3 = G::NXF3, NXFP3 = G::NXFP3, NYF3 = G::NYF3;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* W = reinterpret_cast<T*>(smem_raw);  // [NRING][NV][PL]
   T* SLx = W + NRING * NV * PL;  // [NV][NXS3]; x fluxes in place
@@ -266,7 +315,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
 
   // ---- prologue: planes k0-2 .. k0+1, then the z face k0-1/2 ----
   for (int p = k0 - 2; p <= k0 + 1; ++p)
-    load_plane<T>(a, W, slot(p), p, gi0, gj0, perx, pery, perz, resist, glmf, p == k0);
+    load_plane<T, G>(a, W, slot(p), p, gi0, gj0, perx, pery, perz, resist, glmf, p == k0);
   __syncthreads();
   T sLc[NV];  // z-upper face state of the current cell (k)
   double Fzp[NV] = {};  // z flux through face k-1/2
@@ -282,6 +331,10 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
     }
   }
   double vloc = 0.0;
+  // the FP64 performance build solves all faces in one loop (the FP32 and parity
+  // builds keep a copy of the solver per direction: another component order changes
+  // their rounding)
+  constexpr bool kOneSolver = OMHD_FAST && sizeof(T) == 8;
 
   for (int k = lead_in ? k0 - 1 : k0; k <= k1; ++k) {
     const bool lead = k < k0;  // only the z face k+1/2 (uniform over the CTA)
@@ -331,7 +384,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
         }
       }
       if (k == k0 || seam) __syncthreads();
-      load_plane<T>(a, W, slot(k + 2), k + 2, gi0, gj0, perx, pery, perz, resist, glmf, false);
+      load_plane<T, G>(a, W, slot(k + 2), k + 2, gi0, gj0, perx, pery, perz, resist, glmf, false);
       __syncthreads();
       if (k > k0) {
         // positivity of the current plane's own cells (u2v.f90:36-45); plane k0
@@ -347,7 +400,35 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
       const T* Wk = W + (size_t)slot(k) * NV * PL;
 
       // ---- x and y face states of plane k, one phase ----
-      for (int q = tid; q < NXS3 + NYS3; q += NT) {
+      bool paired = false;
+      if constexpr (kOneSolver) {
+        if (lm == LM_MINMOD || lm == LM_MC) {
+          // two neighbouring cells of a strip per item, their shared slope once
+          paired = true;
+          constexpr int XP = XS / 2, NXP = NXS3 / 2, NYP = NYS3 / 2;
+          static_assert(XS % 2 == 0 && (TY + 2) % 2 == 0, "cell pairs need even strip lengths");
+#pragma unroll 1
+          for (int p = tid; p < NXP + NYP; p += NT) {
+            const bool xd = p < NXP;
+            const int pp = xd ? p : p - NXP;
+            const int ca = xd ? 2 * (pp % XP) : pp % TX, cb = xd ? pp / XP : 2 * (pp / TX);
+            const int o = xd ? (cb + 2) * RX + (ca + 1) : (cb + 1) * RX + (ca + 2);
+            const int st = xd ? 1 : RX, i0 = xd ? cb * XS + ca : cb * TX + ca, di = xd ? 1 : TX;
+            T* dl = xd ? SLx : SLy;
+            T* dr = xd ? SRx : SRy;
+            const int sv = xd ? NXS3 : NYS3;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+              const T* w = Wk + v * PL + o;
+              const T wm = w[-st], w0 = w[0], w1 = w[st], w2 = w[2 * st];
+              const T d0 = w0 - wm, d1 = w1 - w0, d2 = w2 - w1;
+              reconstruct_fp64_g(lm, d0, d1, wm, w0, w1, dl[v * sv + i0], dr[v * sv + i0]);
+              reconstruct_fp64_g(lm, d1, d2, w0, w1, w2, dl[v * sv + i0 + di], dr[v * sv + i0 + di]);
+            }
+          }
+        }
+      }
+      for (int q = tid; !paired && q < NXS3 + NYS3; q += NT) {
         const bool xd = q < NXS3;
         const int qq = xd ? q : q - NXS3;
         int o, st;
@@ -363,7 +444,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
         T* dl = xd ? SLx : SLy;
         T* dr = xd ? SRx : SRy;
         const int sv = xd ? NXS3 : NYS3;
-  #pragma unroll
+#pragma unroll
         for (int v = 0; v < NV; ++v) {
           T l, r;
           reconstruct_t<T, OMHD_FAST>(lm, Wk[v * PL + o - st], Wk[v * PL + o], Wk[v * PL + o + st], l, r);
@@ -405,12 +486,13 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
       // ---- x and y fluxes of plane k, one phase (x faces padded to whole
       // warps, so that no warp mixes directions); each flux replaces the
       // lower-cell face state that only its own face reads ----
+      if constexpr (!kOneSolver)
       for (int q = tid; q < NXFP3 + NYF3; q += NT) {
         if (q < NXFP3) {
           if (q >= NXF3) continue;  // padding lanes
           const int fx = q % XF, cy = q / XF;
           T L[NV], R[NV], Fo[NV];
-  #pragma unroll
+#pragma unroll
           for (int v = 0; v < NV; ++v) {
             L[v] = SLx[v * NXS3 + cy * XS + fx];
             R[v] = SRx[v * NXS3 + cy * XS + fx + 1];
@@ -439,13 +521,13 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
               }
             }
           }
-  #pragma unroll
+#pragma unroll
           for (int v = 0; v < NV; ++v) SLx[v * NXS3 + cy * XS + fx] = Fo[v];
         } else {
           const int qq = q - NXFP3;
           const int cx = qq % TX, fy = qq / TX;
           T L[NV], R[NV], Fo[NV];
-  #pragma unroll
+#pragma unroll
           for (int v = 0; v < NV; ++v) {
             L[v] = SLy[v * NYS3 + fy * TX + cx];
             R[v] = SRy[v * NYS3 + (fy + 1) * TX + cx];
@@ -474,7 +556,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
               }
             }
           }
-  #pragma unroll
+#pragma unroll
           for (int v = 0; v < NV; ++v) SLy[v * NYS3 + fy * TX + cx] = Fo[v];
         }
       }
@@ -530,7 +612,83 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
         }
       }
     };
-    if constexpr (sizeof(T) == 8) z_face();
+    if constexpr (kOneSolver) {
+      // x and y faces of the plane, then this thread's z face k+1/2 (in registers;
+      // it reads only the ring), through one x-oriented solver in one rolled loop:
+      // with a copy per direction a fifth of the warps' time went into instruction
+      // fetches.  Fluxes replace the lower-cell face states that only they read.
+      constexpr int RXY = (NXF3 + NYF3 + NT - 1) / NT;
+#pragma unroll 1
+      for (int r = lead ? RXY : 0; r <= RXY; ++r) {
+        const bool zf = r == RXY;
+        const int q = tid + r * NT, n = zf ? 2 : (q < NXF3 ? 0 : 1);
+        if (!zf && q >= NXF3 + NYF3) continue;
+        const int qq = n == 0 ? q : q - NXF3;
+        const int fa = n == 0 ? qq % XF : qq % TX, fb = n == 0 ? qq / XF : qq / TX;
+        double* const bl = n == 0 ? SLx + fb * XS + fa : SLy + fb * TX + fa;
+        const double* const br = n == 0 ? SRx + fb * XS + fa + 1 : SRy + (fb + 1) * TX + fa;
+        const int sv = n == 0 ? NXS3 : NYS3;
+        double L[NV], R[NV], Fo[NV], F[NV];
+        if (zf) {
+          double Rg[NV];
+#pragma unroll
+          for (int v = 0; v < NV; ++v)
+            reconstruct_t<T, OMHD_FAST>(lm, Wv(k, v, oc), Wv(k + 1, v, oc), Wv(k + 2, v, oc), sLn[v], Rg[v]);
+          if (!perz && k == 0) {  // bottom wall: VL = flip(VR)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) sLc[v] = ((a.bc_flip[4] >> v) & 1) ? -Rg[v] : Rg[v];
+          }
+          if (!perz && k == kx - 2) {  // top wall: VR = flip(VL)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) Rg[v] = ((a.bc_flip[5] >> v) & 1) ? -sLc[v] : sLc[v];
+          }
+#pragma unroll
+          for (int c = 0; c < NV; ++c) {
+            L[c] = sLc[rot3(2, c)];
+            R[c] = Rg[rot3(2, c)];
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < NV; ++c) {
+            const int pv = (n == 0 ? c : rot3(1, c)) * sv;
+            L[c] = bl[pv];
+            R[c] = br[pv];
+          }
+        }
+        riemann_flux<double, 1, FLUX, true>(L, R, ch, gam, r1, r2, Fo);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {  // back to grid components: v = rot3(1, rot3(2, v)) = rot3(2, rot3(1, v))
+          F[v] = n == 0 ? Fo[v] : (n == 1 ? Fo[rot3(2, v)] : Fo[rot3(1, v)]);
+        }
+        if (resist) {
+          const int gx = zf ? gi : (n == 0 ? gi0 - 1 + fa : gi0 + fa), gy = zf ? gj : (n == 0 ? gj0 + fb : gj0 - 1 + fb);
+          if (gx >= 0 && gy >= 0 && gx <= ix - 2 && gy <= jx - 2) {
+            const int o = zf ? oc : (n == 0 ? (fb + 2) * RX + (fa + 1) : (fb + 1) * RX + (fa + 2));
+            const int ex_i = zf ? tx + 1 : (n == 0 ? fa : fa + 1);
+            auto B = [&](int var, int dxo, int dyo, int dzo) { return Wv(k + dzo, var, o + dxo + dyo * RX); };
+            const double eta_dx =
+                sep_eta ? harris_eta_dx<double>((n == 0 ? ex_f : ex_c)[ex_i], (zf ? ez_f : ez_c)[k - k0 + 1], inv_dx)
+                        : eta3(a.eta_kind, a.xc[gx] + (n == 0 ? 0.5 * a.dx : 0.0), a.yc[gy] + (n == 1 ? 0.5 * a.dx : 0.0),
+                               a.zc[k] + (zf ? 0.5 * a.dx : 0.0)) / a.dx;
+            if (zf)
+              resist_face_f64<2>(B, eta_dx, F);
+            else if (n == 0)
+              resist_face_f64<0>(B, eta_dx, F);
+            else
+              resist_face_f64<1>(B, eta_dx, F);
+          }
+        }
+        if (zf) {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) Fzc[v] = F[v];
+        } else {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) bl[v * sv] = F[v];
+        }
+      }
+    } else if constexpr (sizeof(T) == 8) {
+      z_face();
+    }
 
     double acc[NV] = {}, gm[NV] = {}, gp[NV] = {};
     if (!lead) {
@@ -633,21 +791,47 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 
   }
 }
 
-template <class T, int FLUX>
-int launch_one3d(const StageArgs& a, cudaStream_t s) {
-  const size_t bytes = smem3d_bytes<T>();
-  static std::atomic<unsigned long long> configured{0};
-  const int r = set_smem_attr_once(k_stage3d<T, FLUX>, bytes, configured);
-  if (r) return r;
-  int dev = 0, nsm = 0;
+inline int sm_count(int* nsm) {
+  int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return (int)e;
-  dim3 grid((a.ix - 2 + TX - 1) / TX, (a.jx - 2 + TY - 1) / TY, 1);
-  const int zc = pick_zchunk((long long)grid.x * grid.y, a.kx - 2, nsm * (sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 1));
-  grid.z = (a.kx - 2 + zc - 1) / zc;
-  k_stage3d<T, FLUX><<<grid, NT, bytes, s>>>(a, zc);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev);
+  return (int)e;
+}
+
+template <class G>
+inline long long columns_of(const StageArgs& a) {
+  return (long long)((a.ix - 2 + G::TX - 1) / G::TX) * ((a.jx - 2 + G::TY - 1) / G::TY);
+}
+
+template <class T, int FLUX, class G = DefaultCol<T>>
+int launch_one3d(const StageArgs& a, cudaStream_t s) {
+  const size_t bytes = G::template smem_bytes<T>();
+  static std::atomic<unsigned long long> configured{0};
+  int r = set_smem_attr_once(k_stage3d<T, FLUX, G>, bytes, configured);
+  int nsm = 0;
+  if (!r) r = sm_count(&nsm);
+  if (r) return r;
+  const int zc = pick_zchunk(columns_of<G>(a), a.kx - 2, nsm * G::CTAS);
+  dim3 grid((a.ix - 2 + G::TX - 1) / G::TX, (a.jx - 2 + G::TY - 1) / G::TY, (a.kx - 2 + zc - 1) / zc);
+  k_stage3d<T, FLUX, G><<<grid, G::NT, bytes, s>>>(a, zc);
   return (int)cudaGetLastError();
+}
+
+// FP64 HLLD: 16x16 columns, one CTA per SM, or two CTAs of 16x8 columns, the
+// cheaper by the rounds x (planes + prologue) of pick_zchunk; an SM takes 7 %
+// longer for a plane of two 16x8 columns, whose halo is larger (Harris
+// 256x128x256, ms per step: 33.4 with 16x16, 35.9 with 16x8, 34.0 with 32x8), but
+// covers ragged grids better (field loop 100x100x200: 6.5, 5.7, 7.2).
+template <int FLUX>
+int launch_best3d(const StageArgs& a, cudaStream_t s) {
+  int nsm = 0;
+  const int r = sm_count(&nsm);
+  if (r) return r;
+  double wide = 0.0, small = 0.0;
+  pick_zchunk(columns_of<WideCol>(a), a.kx - 2, nsm * WideCol::CTAS, &wide);
+  pick_zchunk(columns_of<SmallCol>(a), a.kx - 2, nsm * SmallCol::CTAS, &small);
+  if (1.07 * small < wide) return launch_one3d<double, FLUX, SmallCol>(a, s);
+  return launch_one3d<double, FLUX, WideCol>(a, s);
 }
 
 template <class T>
@@ -656,7 +840,11 @@ int launch_variant3d(const StageArgs& a, cudaStream_t s) {
     case FX_LLF: return launch_one3d<T, FX_LLF>(a, s);
     case FX_HLL: return launch_one3d<T, FX_HLL>(a, s);
     case FX_HLLC: return launch_one3d<T, FX_HLLC>(a, s);
-    case FX_HLLD: return launch_one3d<T, FX_HLLD>(a, s);
+    case FX_HLLD:
+      if constexpr (OMHD_FAST && sizeof(T) == 8)
+        return launch_best3d<FX_HLLD>(a, s);
+      else
+        return launch_one3d<T, FX_HLLD>(a, s);
     default: return launch_one3d<T, FX_LHLLD>(a, s);
   }
 }
