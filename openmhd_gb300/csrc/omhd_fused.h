@@ -24,6 +24,10 @@ struct StageArgs {
   int lm_type, flux_type, time_type, stage, iso;
   int bc_kind[6], bc_flip[6];
   int eta_kind;
+  // eta/dx at the x and y faces of a 2D resistive grid, indexed by the face's lower
+  // cell (fill_eta2d_*), or nullptr: evaluated per face and stage
+  const double* etax;
+  const double* etay;
   const double* xc;     // cell-centre coordinates (resistive runs)
   const double* yc;
   const double* zc;
@@ -68,6 +72,10 @@ inline void stage_args_derived(StageArgs& a) {
 int launch_stage2d_fp64(const StageArgs& a, cudaStream_t s);
 int launch_stage2d_parity(const StageArgs& a, cudaStream_t s);
 int launch_stage2d_mixed(const StageArgs& a, cudaStream_t s);
+// eta/dx of the faces of the 2D grid described by a, ix*jx values each
+int fill_eta2d_fp64(const StageArgs& a, double* etax, double* etay, cudaStream_t s);
+int fill_eta2d_parity(const StageArgs& a, double* etax, double* etay, cudaStream_t s);
+int fill_eta2d_mixed(const StageArgs& a, double* etax, double* etay, cudaStream_t s);
 // fp64 HLLD stage with a decision tape: mode tape::kRecord or tape::kReplay
 int launch_stage2d_fp64_tape(const StageArgs& a, int mode, cudaStream_t s);
 // ensemble launchers: tile_kind 0: 32x8, 1: 32x4, 2: 16x16, 3: 64x4, 4: 16x8 cells per CTA

@@ -106,6 +106,34 @@ __device__ __forceinline__ double eta_at(int kind, double x, double y, double z)
   return 0.0;
 }
 
+// eta/dx of the x face between cells g and g+1 of row j, and of the y face between
+// rows g and g+1 of column i.  The profile does not change in time, and its cosh is
+// as much FP64 work as a face's Riemann solver: a solver tabulates it once
+// (16 bytes a cell, read beside the 360 of a step).
+__device__ __forceinline__ double eta_x(const StageArgs& a, int g, int j) {
+  if (a.etax) return __ldg(a.etax + (size_t)g + (size_t)a.ix * j);
+  const double odx = 1.0 / a.dx;
+  return eta_at(a.eta_kind, a.xc[g] + 0.5 * a.dx, a.yc[j], 0.0) * odx;
+}
+__device__ __forceinline__ double eta_y(const StageArgs& a, int i, int g) {
+  if (a.etay) return __ldg(a.etay + (size_t)i + (size_t)a.ix * g);
+  const double odx = 1.0 / a.dx;
+  return eta_at(a.eta_kind, a.xc[i], a.yc[g] + 0.5 * a.dx, 0.0) * odx;
+}
+__global__ void k_eta2d(StageArgs a, double* __restrict__ etax, double* __restrict__ etay) {
+  a.etax = a.etay = nullptr;
+  const size_t n = (size_t)a.ix * a.jx;
+  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
+    const int i = (int)(c % a.ix), j = (int)(c / a.ix);
+    etax[c] = eta_x(a, i, j);
+    etay[c] = eta_y(a, i, j);
+  }
+}
+inline int fill_eta2d(const StageArgs& a, double* etax, double* etay, cudaStream_t s) {
+  k_eta2d<<<1216, 128, 0, s>>>(a, etax, etay);
+  return (int)cudaGetLastError();
+}
+
 // canonical interior cell of a (possibly ghost or out-of-grid) index along an
 // axis of extent n, for decision-tape lookups: periodic ghosts wrap, other
 // indices clamp (their states are unused)
@@ -124,9 +152,14 @@ __device__ __forceinline__ int tape_cell(int g, int n, bool periodic) {
 // own FP64 block (FX[v*fxv + cy*(TX+1) + fx], FY[v*fyv + fy*TX + cx]) or, in
 // the FP64 pipelined kernel, overwrite the lower-cell face state that only
 // their own face reads (FX = SLx with fxv = NXS and row stride TX+2).
+// Bf: the cell-centred field components the resistive terms read, three planes: in
+// W, or (pipelined kernel) a copy of the tile's own that phase_load fills (bcopy),
+// because the producers refill W while the consumers solve the faces.
 template <class T>
 struct TileMem {
   T* W;
+  const T* Bf;
+  T* bcopy;
   T *SLx, *SRx, *SLy, *SRy;
   double *FX, *FY;
   int fxv, fxr, fyv;
@@ -175,6 +208,8 @@ template <class T, class G>
 __device__ __forceinline__ TileMem<T> tile_mem_separate(unsigned char* smem_raw) {
   TileMem<T> m;
   m.W = reinterpret_cast<T*>(smem_raw);
+  m.Bf = m.W + BX * G::RX * G::RY;
+  m.bcopy = nullptr;
   m.SLx = m.W + NV * G::RX * G::RY;
   m.SRx = m.SLx + NV * G::NXS;
   m.SLy = m.SRx + NV * G::NXS;
@@ -245,6 +280,10 @@ __device__ __forceinline__ void phase_load(const StageArgs& a, int bxi, int byi,
       u2v_cell<T, OMHD_FAST>(u[b], f1g, f1g32, ps, w, pr, ro);
 #pragma unroll
       for (int v = 0; v < NV; ++v) W[v * PL + q] = w[v];
+      if (m.bcopy) {
+#pragma unroll
+        for (int v = 0; v < 3; ++v) m.bcopy[v * PL + q] = w[BX + v];
+      }
       if (cx_in && cy_in && gi <= ix - 2 && gj <= jx - 2) {  // owner check, u2v.f90:36-45
         if (!gt0_<OMHD_FAST>(pr))
           raise_error(a.err, OMHD_NEG_PRESSURE, gi + 1, gj + 1, 0, 0, pr);
@@ -455,7 +494,6 @@ __device__ __forceinline__ void phase_flux_rot(const StageArgs& a, int bxi, int 
   const int gi0 = 1 + bxi * TX, gj0 = 1 + byi * ty;
   const bool resist = a.eta_kind != OMHD_ETA_NONE;
   const T ch = ks.ch, gam = ks.gam, r1 = ks.r1, r2 = ks.r2;
-  const T* W = m.W;
 #pragma unroll 1
   for (int q = t; q < nxf + nyf; q += n) {
     const bool xd = q < nxf;
@@ -500,9 +538,8 @@ __device__ __forceinline__ void phase_flux_rot(const StageArgs& a, int bxi, int 
         const int fx = fa, cy = fb, g = gi0 - 1 + fx, gj = gj0 + cy;
         if (g >= 0 && g <= ix - 2 && gj <= jx - 2) {
           const int o = (cy + 2) * RX + (fx + 1);  // region index of cell g
-          auto B = [&](int var, int dxo, int dyo) { return to_f64<T>(W[var * PL + o + dxo + dyo * RX]); };
-          const double odx = 1.0 / a.dx;
-          const double eta_dx = eta_at(a.eta_kind, a.xc[g] + 0.5 * a.dx, a.yc[gj], 0.0) * odx;
+          auto B = [&](int var, int dxo, int dyo) { return to_f64<T>(m.Bf[(var - BX) * PL + o + dxo + dyo * RX]); };
+          const double eta_dx = eta_x(a, g, gj);
           const double JyS = -eta_dx * (B(BZ, 1, 0) - B(BZ, 0, 0));
           const double JzS = eta_dx * ((B(BY, 1, 0) - B(BY, 0, 0)) -
                                        0.25 * (B(BX, 0, 1) + B(BX, 1, 1) - B(BX, 0, -1) - B(BX, 1, -1)));
@@ -514,9 +551,8 @@ __device__ __forceinline__ void phase_flux_rot(const StageArgs& a, int bxi, int 
         const int cx = fa, fy = fb, gi = gi0 + cx, g = gj0 - 1 + fy;
         if (g >= 0 && g <= jx - 2 && gi <= ix - 2) {
           const int o = (fy + 1) * RX + (cx + 2);  // region index of cell (gi, g)
-          auto B = [&](int var, int dxo, int dyo) { return to_f64<T>(W[var * PL + o + dxo + dyo * RX]); };
-          const double odx = 1.0 / a.dx;
-          const double eta_dx = eta_at(a.eta_kind, a.xc[gi], a.yc[g] + 0.5 * a.dx, 0.0) * odx;
+          auto B = [&](int var, int dxo, int dyo) { return to_f64<T>(m.Bf[(var - BX) * PL + o + dxo + dyo * RX]); };
+          const double eta_dx = eta_y(a, gi, g);
           const double JxS = eta_dx * (B(BZ, 0, 1) - B(BZ, 0, 0));
           const double JzS = eta_dx * (0.25 * (B(BY, 1, 1) + B(BY, 1, 0) - B(BY, -1, 1) - B(BY, -1, 0)) -
                                        (B(BX, 0, 1) - B(BX, 0, 0)));
@@ -578,8 +614,7 @@ __device__ __forceinline__ void phase_flux(const StageArgs& a, int bxi, int byi,
         if (g >= 0 && g <= ix - 2 && gj <= jx - 2) {
           const int o = (cy + 2) * RX + (fx + 1);  // region index of cell g
           auto B = [&](int var, int dxo, int dyo) { return to_f64<T>(W[var * PL + o + dxo + dyo * RX]); };
-          const double odx = 1.0 / a.dx;
-          const double eta_dx = eta_at(a.eta_kind, a.xc[g] + 0.5 * a.dx, a.yc[gj], 0.0) * odx;
+          const double eta_dx = eta_x(a, g, gj);
           const double JyS = -eta_dx * (B(BZ, 1, 0) - B(BZ, 0, 0));
           const double JzS = eta_dx * ((B(BY, 1, 0) - B(BY, 0, 0)) -
                                        0.25 * (B(BX, 0, 1) + B(BX, 1, 1) - B(BX, 0, -1) - B(BX, 1, -1)));
@@ -614,8 +649,7 @@ __device__ __forceinline__ void phase_flux(const StageArgs& a, int bxi, int byi,
         if (g >= 0 && g <= jx - 2 && gi <= ix - 2) {
           const int o = (fy + 1) * RX + (cx + 2);  // region index of cell (gi, g)
           auto B = [&](int var, int dxo, int dyo) { return to_f64<T>(W[var * PL + o + dxo + dyo * RX]); };
-          const double odx = 1.0 / a.dx;
-          const double eta_dx = eta_at(a.eta_kind, a.xc[gi], a.yc[g] + 0.5 * a.dx, 0.0) * odx;
+          const double eta_dx = eta_y(a, gi, g);
           const double JxS = eta_dx * (B(BZ, 0, 1) - B(BZ, 0, 0));
           const double JzS = eta_dx * (0.25 * (B(BY, 1, 1) + B(BY, 1, 0) - B(BY, -1, 1) - B(BY, -1, 0)) -
                                        (B(BX, 0, 1) - B(BX, 0, 0)));
@@ -810,8 +844,10 @@ __global__ void __launch_bounds__(GeoFor<T>::type::NT, sizeof(T) == 4 ? OMHD_MIX
 // W + 2 buffers = 195 KB.  Tiles are 16 cells wide and ty <= 16 rows high
 // (pick_rows); the loops over a tile run to ty, which also keeps them rolled: the
 // unrolled flux loop (two copies of the solver) cost 8 % in instruction fetches.
-// Non-resistive 2D runs (the resistive terms read W in phase C, which the
-// producers already refill).
+// In resistive runs the TMA staging area holds a copy of each buffer's field
+// components, which the resistive terms read in phase C while the producers
+// already refill W (reconnection 500x125, 5 steps: 1.16 ms in the one-role kernel
+// with eta evaluated per face).
 // Measured on KH 4096x2048, ms per step: 20.3 with the FP64-pipe arithmetic, 17.7
 // with integer reciprocals and roots, 14.1 with integer products, 12.9 rolled and
 // with the CFL bound; FP64 pipe 76 % busy (84 % is all it gives with 12 warps).
@@ -836,16 +872,19 @@ constexpr unsigned kPipeBoxBytes = sizeof(double) * NV * kPipeBoxX * kPipeBoxY;
 constexpr size_t pipe_stage_off() { return (pipe_smem_bytes() + 127) / 128 * 128; }
 constexpr size_t pipe_smem_bytes_tma() { return pipe_stage_off() + 128 + kPipeBoxBytes; }
 static_assert(pipe_smem_bytes_tma() <= 232448 - 512, "pipelined kernel exceeds the shared memory of one CTA");
+static_assert(2 * 3 * sizeof(double) * PipeGeo::RX * PipeGeo::RY <= kPipeBoxBytes, "the field copies fit the staging area");
 static_assert((kPipeBoxX * 8) % 16 == 0, "TMA box rows must be whole 16-byte units");
 // polls of a TMA completion before a tile is declared lost (well beyond any
 // real transfer; the kernel then records OMHD_TIMEOUT and keeps its barrier
 // protocol, so nothing waits forever)
 constexpr uint32_t kTmaMaxPolls = 1u << 22;
 
-__device__ __forceinline__ TileMem<double> pipe_mem(unsigned char* smem_raw, int b) {
+__device__ __forceinline__ TileMem<double> pipe_mem(unsigned char* smem_raw, int b, bool resist) {
   using G = PipeGeo;
   TileMem<double> m;
   m.W = reinterpret_cast<double*>(smem_raw);
+  m.bcopy = resist ? reinterpret_cast<double*>(smem_raw + pipe_stage_off()) + (size_t)b * 3 * G::RX * G::RY : nullptr;
+  m.Bf = m.bcopy;
   m.SLx = m.W + NV * G::RX * G::RY + (size_t)b * NV * 2 * (G::NXS + G::NYS);
   m.SRx = m.SLx + NV * G::NXS;
   m.SLy = m.SRx + NV * G::NXS;
@@ -876,6 +915,7 @@ __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
   __syncthreads();
   if (skip) return;
   const double glmf = ks.glmf;
+  const bool resist = a.eta_kind != OMHD_ETA_NONE;  // then the staging area holds the field copies (use_tma = 0)
   const int ntx = (a.ix - 2 + G::TX - 1) / G::TX;
   const int ntiles = ntx * ((a.jx - 2 + ty - 1) / ty);
   double vmax = 0.0;
@@ -903,7 +943,7 @@ __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
   const int wfirst = blockIdx.x, wsecond = wfirst + (int)gridDim.x;
   {
     if (use_tma && threadIdx.x == 0) mbar_init(&tma_bar, 1);
-    const TileMem<double> m = pipe_mem(smem_raw, 0);
+    const TileMem<double> m = pipe_mem(smem_raw, 0, resist);
     phase_load<double, G>(a, wfirst % ntx, wfirst / ntx, m, threadIdx.x, NTOT, glmf, nullptr, ty);
     __syncthreads();
     if (threadIdx.x == 0 && wsecond < ntiles && staged(wsecond)) issue(wsecond);
@@ -921,7 +961,7 @@ __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
     int i = 1;
     for (int w = wsecond; w < ntiles; w += gridDim.x, ++i) {
       const int b = i & 1;
-      const TileMem<double> m = pipe_mem(smem_raw, b);
+      const TileMem<double> m = pipe_mem(smem_raw, b, resist);
       if (i >= 2) named_bar_sync(kPipeBarEmpty + b, NTOT);  // consumers are done with buffer b
       if (i >= 2) named_bar_sync(kPipeBarProd, NP);         // W of the previous tile is read
       if (staged(w) && !tma_lost) {
@@ -952,7 +992,7 @@ __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
     int i = 0;
     for (int w = blockIdx.x; w < ntiles; w += gridDim.x, ++i) {
       const int b = i & 1;
-      const TileMem<double> m = pipe_mem(smem_raw, b);
+      const TileMem<double> m = pipe_mem(smem_raw, b, resist);
       if (i >= 1) named_bar_sync(kPipeBarFull + b, NTOT);
       const float known = a.stage == 2 ? cfl_known(st) : 0.0f;
       phase_flux<double, FLUX, G, TAPE>(a, w % ntx, w / ntx, m, t, NC, ks, ty);
@@ -1019,7 +1059,7 @@ int launch_pipe(const StageArgs& a, cudaStream_t s) {
   CUtensorMap tmap;
   memset(&tmap, 0, sizeof tmap);
   const int use_tma =
-      tma_staging_enabled() && tma_encode_state_map(&tmap, a.Uin, a.ix, a.jx, NV, kPipeBoxX, kPipeBoxY) == 0;
+      a.eta_kind == OMHD_ETA_NONE && tma_staging_enabled() && tma_encode_state_map(&tmap, a.Uin, a.ix, a.jx, NV, kPipeBoxX, kPipeBoxY) == 0;
   k_stage2d_pipe<FLUX, TAPE, NPW><<<grid, NPW * 32 + PipeGeo::NT, bytes, s>>>(a, tmap, use_tma, ty);
   return (int)cudaGetLastError();
 }

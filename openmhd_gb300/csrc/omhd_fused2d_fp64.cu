@@ -5,6 +5,9 @@
 #include "omhd_fused2d.cuh"
 
 namespace omhd {
+int fill_eta2d_fp64(const StageArgs& a, double* etax, double* etay, cudaStream_t s) {
+  return v_fp64::fill_eta2d(a, etax, etay, s);
+}
 // HLLD with minmod or MC runs the tape-recording instantiation with recording
 // switched off (null tape pointers): one machine code for the plain and the
 // recording step, so a recorded run reproduces a plain run bit for bit.
@@ -13,7 +16,7 @@ int launch_stage2d_fp64(const StageArgs& a, cudaStream_t s) {
     StageArgs b = a;
     b.tlim = nullptr;
     b.tface = nullptr;
-    if (a.eta_kind == OMHD_ETA_NONE && pipe2d_enabled())
+    if (pipe2d_enabled())
       return v_fp64::launch_pipe<FX_HLLD, tape::kRecord>(b, s);
     return v_fp64::launch_one<double, FX_HLLD, tape::kRecord>(b, s);
   }
@@ -23,8 +26,7 @@ int launch_stage2d_fp64_tape(const StageArgs& a, int mode, cudaStream_t s) {
   if (a.flux_type != FX_HLLD || a.nd != 2 || !a.tlim || !a.tface) return (int)cudaErrorInvalidValue;
   if (a.lm_type != LM_MINMOD && a.lm_type != LM_MC) return (int)cudaErrorInvalidValue;
   if (mode == tape::kRecord) {
-    if (a.eta_kind == OMHD_ETA_NONE) return v_fp64::launch_pipe<FX_HLLD, tape::kRecord>(a, s);
-    return v_fp64::launch_one<double, FX_HLLD, tape::kRecord>(a, s);
+    return v_fp64::launch_pipe<FX_HLLD, tape::kRecord>(a, s);
   }
   if (mode == tape::kReplay) return v_fp64::launch_one<double, FX_HLLD, tape::kReplay>(a, s);
   return (int)cudaErrorInvalidValue;

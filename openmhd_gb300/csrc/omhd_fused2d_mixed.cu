@@ -5,6 +5,9 @@
 #include "omhd_fused2d.cuh"
 
 namespace omhd {
+int fill_eta2d_mixed(const StageArgs& a, double* etax, double* etay, cudaStream_t s) {
+  return v_mixed::fill_eta2d(a, etax, etay, s);
+}
 int launch_stage2d_mixed(const StageArgs& a, cudaStream_t s) { return v_mixed::launch_variant<float>(a, s); }
 }  // namespace omhd
 

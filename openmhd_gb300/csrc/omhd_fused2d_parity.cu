@@ -5,5 +5,8 @@
 #include "omhd_fused2d.cuh"
 
 namespace omhd {
+int fill_eta2d_parity(const StageArgs& a, double* etax, double* etay, cudaStream_t s) {
+  return v_parity::fill_eta2d(a, etax, etay, s);
+}
 int launch_stage2d_parity(const StageArgs& a, cudaStream_t s) { return v_parity::launch_variant<double>(a, s); }
 }  // namespace omhd

@@ -285,6 +285,8 @@ StageArgs make_stage_args(const omhd_solver* s, int stage) {
     a.bc_flip[q] = c.bc_flip[q];
   }
   a.eta_kind = c.eta_kind;
+  a.etax = s->eta;
+  a.etay = s->eta ? s->eta + s->n : nullptr;
   a.xc = s->xc;
   a.yc = s->yc;
   a.zc = s->zc;
@@ -393,6 +395,24 @@ int plan_first(omhd_solver* s, double t) {
   return cerr(s, cudaGetLastError(), "cfl kernel");
 }
 
+// eta/dx at the faces of a resistive 2D grid, in the variant's own arithmetic; where
+// there is no memory for the tables the kernels evaluate it per face
+int tabulate_eta(omhd_solver* s) {
+  double* t = nullptr;
+  if (cudaMalloc(&t, sizeof(double) * 2 * s->n) != cudaSuccess) {
+    cudaGetLastError();
+    return OMHD_OK;
+  }
+  const StageArgs a = make_stage_args(s, 1);
+  const int p = s->cfg.precision;
+  const int e = p == OMHD_PREC_FP64          ? fill_eta2d_fp64(a, t, t + s->n, nullptr)
+                : p == OMHD_PREC_FP64_PARITY ? fill_eta2d_parity(a, t, t + s->n, nullptr)
+                                             : fill_eta2d_mixed(a, t, t + s->n, nullptr);
+  s->eta = t;
+  const int r = cerr(s, (cudaError_t)e, "eta table kernel");
+  return r ? r : cerr(s, cudaStreamSynchronize(nullptr), "eta table");
+}
+
 void drop_graph(omhd_solver* s) {
   if (s->graph) cudaGraphExecDestroy(s->graph);
   s->graph = nullptr;
@@ -443,6 +463,7 @@ int omhd_solver_create(const omhd_config* cfg, omhd_solver** out) {
     cudaMemset(s->st, 0, sizeof(StepState));
     cudaMemset(s->err, 0, sizeof(DevError));
   }
+  if (!r && c.nd == 2 && c.eta_kind != OMHD_ETA_NONE) r = tabulate_eta(s);
   if (r) {
     omhd_solver_destroy(s);
     return r;
@@ -461,6 +482,7 @@ int omhd_solver_destroy(omhd_solver* s) {
   cudaFree(s->xc);
   cudaFree(s->yc);
   cudaFree(s->zc);
+  cudaFree(s->eta);
   cudaFree(s->st);
   cudaFree(s->err);
   delete s;

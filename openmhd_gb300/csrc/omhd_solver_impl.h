@@ -22,6 +22,7 @@ struct omhd_solver {
   double* xc = nullptr;  // device coordinates
   double* yc = nullptr;
   double* zc = nullptr;
+  double* eta = nullptr;  // 2D resistive grids: eta/dx at the x faces, then at the y faces
   std::vector<double> hx, hy, hz;
   omhd::StepState* st = nullptr;
   omhd::DevError* err = nullptr;
