@@ -65,19 +65,28 @@ __device__ __forceinline__ bool lt_(T a, T b) {  // a < b
 template <class T, bool FAST, bool FPIPE = false>
 __device__ __forceinline__ T rcp_(T b) {
   if constexpr (FAST && sizeof(T) == 8) return FPIPE ? rcp_nr_fp(b) : rcp_nr(b);
+  if constexpr (sizeof(T) == 8) return div_rn(1.0, b);
   return T(1) / b;
 }
 template <class T, bool FAST>
 __device__ __forceinline__ T div_(T a, T b) {
   if constexpr (FAST && sizeof(T) == 8) return a * rcp_nr(b);
+  if constexpr (sizeof(T) == 8) return div_rn(a, b);
   return a / b;
+}
+// the IEEE square root, on the integer pipes in the FP64 kernels that keep the
+// reference's operations
+template <class T, bool FAST>
+__device__ __forceinline__ T sqrt_x(T x) {
+  if constexpr (!FAST && sizeof(T) == 8) return sqrt_rn(x);
+  return sqrt(x);
 }
 // square root under the variant's policy: sqrt_nr for FAST FP64 (IEEE outside the
 // positive normal range, so sqrt(+-0) = +-0)
 template <class T, bool FAST, bool FPIPE = false>
 __device__ __forceinline__ T sqrt_(T x) {
   if constexpr (FAST && sizeof(T) == 8) return FPIPE ? sqrt_nr_fp(x) : sqrt_nr(x);
-  return sqrt(x);
+  return sqrt_x<T, FAST>(x);
 }
 // sqrt(a / b) for a, b > 0: a * (1/sqrt(a*b)) for FAST FP64 (one product and
 // one rsqrt refinement replace a division and a square root), IEEE otherwise
@@ -87,13 +96,13 @@ __device__ __forceinline__ T sqrt_ratio_(T a, T b) {
     const double ab = a * b;
     return pos_normal(ab) ? a * (FPIPE ? rsqrt_nr_fp(ab) : rsqrt_nr(ab)) : sqrt(a / b);
   }
-  return sqrt(a / b);
+  return sqrt_x<T, FAST>(div_<T, FAST>(a, b));
 }
 // a / b given rb = rcp_<T,FAST>(b) computed once for several numerators
 template <class T, bool FAST>
 __device__ __forceinline__ T divr_(T a, T b, T rb) {
   if constexpr (FAST && sizeof(T) == 8) return a * rb;
-  return a / b;
+  return div_<T, FAST>(a, b);
 }
 
 // primitive (FP64) -> the face arithmetic's type T, and face flux -> FP64: the
@@ -610,7 +619,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
   f1 = gamma * L[PR];
   f2 = 4 * (L[bn] * L[bn]);
   if (TYPE == FX_LLF) {
-    aL = sqrt(div_<T, FAST>((f1 + B2) + sqrt((f1 + B2) * (f1 + B2) - f1 * f2), 2 * L[RO]));
+    aL = sqrt_x<T, FAST>(div_<T, FAST>((f1 + B2) + sqrt_x<T, FAST>((f1 + B2) * (f1 + B2) - f1 * f2), 2 * L[RO]));
   } else {
     {  // fmax2(D, 0)
       const T D = (f1 + B2) * (f1 + B2) - f1 * f2;
@@ -620,7 +629,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
     ptL = L[PR] + T(0.5) * B2;
     if (TYPE == FX_LHLLD) {
       const T g1 = L[RO] * v2;
-      aL1 = div_<T, FAST>((g1 + B2) + sqrt(fmax2((g1 + B2) * (g1 + B2) - g1 * f2, T(0))), 2 * L[RO]);
+      aL1 = div_<T, FAST>((g1 + B2) + sqrt_x<T, FAST>(fmax2((g1 + B2) * (g1 + B2) - g1 * f2, T(0))), 2 * L[RO]);
     }
   }
 
@@ -642,7 +651,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
   f1 = gamma * R[PR];
   f2 = 4 * (R[bn] * R[bn]);
   if (TYPE == FX_LLF) {
-    aR = sqrt(div_<T, FAST>((f1 + B2) + sqrt((f1 + B2) * (f1 + B2) - f1 * f2), 2 * R[RO]));
+    aR = sqrt_x<T, FAST>(div_<T, FAST>((f1 + B2) + sqrt_x<T, FAST>((f1 + B2) * (f1 + B2) - f1 * f2), 2 * R[RO]));
   } else {
     {  // fmax2(D, 0)
       const T D = (f1 + B2) * (f1 + B2) - f1 * f2;
@@ -652,7 +661,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
     ptR = R[PR] + T(0.5) * B2;
     if (TYPE == FX_LHLLD) {
       const T g1 = R[RO] * v2;
-      aR1 = div_<T, FAST>((g1 + B2) + sqrt(fmax2((g1 + B2) * (g1 + B2) - g1 * f2, T(0))), 2 * R[RO]);
+      aR1 = div_<T, FAST>((g1 + B2) + sqrt_x<T, FAST>(fmax2((g1 + B2) * (g1 + B2) - g1 * f2, T(0))), 2 * R[RO]);
     }
   }
 
@@ -664,7 +673,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
     Fo[bt1] = T(0.5) * (FL[bt1] + FR[bt1] - f1 * (R[bt1] - L[bt1]));
     Fo[bt2] = T(0.5) * (FL[bt2] + FR[bt2] - f1 * (R[bt2] - L[bt2]));
   } else if (TYPE == FX_HLL) {  // :205-214
-    f1 = sqrt(fmax2(aL, aR));
+    f1 = sqrt_x<T, FAST>(fmax2(aL, aR));
     aL = fmin2(fmin2(L[vn], R[vn]) - f1, T(0));
     aR = fmax2(fmax2(L[vn], R[vn]) + f1, T(0));
     f1 = rcp_<T, FAST>(aR - aL);
@@ -676,7 +685,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
     Fo[bt2] = f1 * (aR * FL[bt2] - aL * FR[bt2] + f2 * (R[bt2] - L[bt2]));
   } else if (TYPE == FX_HLLC) {  // :281-340
     T Uh[NV];
-    f1 = sqrt(fmax2(aL, aR));
+    f1 = sqrt_x<T, FAST>(fmax2(aL, aR));
     aL = fmin2(fmin2(L[vn], R[vn]) - f1, T(0));
     aR = fmax2(fmax2(L[vn], R[vn]) + f1, T(0));
     f1 = rcp_<T, FAST>(aR - aL);
@@ -709,7 +718,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
     T psi = T(0);
     if (TYPE == FX_LHLLD) {
       f1 = fmin2(T(1), div_<T, FAST>(fmax2(aL1, aR1), fmax2(aL, aR)));
-      psi = 2 * sqrt(f1) - f1;
+      psi = 2 * sqrt_x<T, FAST>(f1) - f1;
     }
     f1 = sqrt_<T, FAST>(decide<TAPE>(lt_<T, FAST>(aL, aR), code, tape::kArSel) ? aR : aL);  // fmax2(aL, aR)
     aL = (decide<TAPE>(lt_<T, FAST>(R[vn], L[vn]), code, tape::kMinR) ? R[vn] : L[vn]) - f1;  // fmin2
@@ -741,7 +750,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
       const T ieR = (FAST && sizeof(T) == 8) ? rcp_<T, FAST>(aR - aM) : T(0);
       const T roL = divr_<T, FAST>(L[RO] * (aL - L[vn]), aL - aM, ieL);
       const T roR = divr_<T, FAST>(R[RO] * (aR - R[vn]), aR - aM, ieR);
-      // Alfven speeds; the FAST variant keeps 1/sqrt(rho*) for the central states
+      // Alfven speeds; the FAST variant keeps 1/sqrt_x<T, FAST>(rho*) for the central states
       T rsL = T(0), rsR = T(0);
       if constexpr (FAST && sizeof(T) == 8) {
         rsL = rsqrt_nr(roL);
@@ -750,8 +759,8 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
       // |Bn| and sign(1, Bn) from one recorded sign bit under a tape
       const bool bneg = decide<TAPE>(signbit(Uh[bn]) != 0, code, tape::kBnNeg);
       const T aBn = (TAPE == tape::kNone) ? fabs(Uh[bn]) : (bneg ? -Uh[bn] : Uh[bn]);
-      const T aVL = (FAST && sizeof(T) == 8) ? aBn * rsL : aBn / sqrt(roL);
-      const T aVR = (FAST && sizeof(T) == 8) ? aBn * rsR : aBn / sqrt(roR);
+      const T aVL = (FAST && sizeof(T) == 8) ? aBn * rsL : div_<T, FAST>(aBn, sqrt_x<T, FAST>(roL));
+      const T aVR = (FAST && sizeof(T) == 8) ? aBn * rsR : div_<T, FAST>(aBn, sqrt_x<T, FAST>(roR));
       if (TYPE == FX_HLLD && decide<TAPE>(!lt_<T, FAST>(aL, aM - hllg_factor * aVL) ||
                                               !lt_<T, FAST>(aM + hllg_factor * aVR, aR),
                                           code, tape::kG)) {
@@ -830,8 +839,8 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
           Fo[bt2] = aR * (UR1[bt2] - R[bt2]) + FR[bt2];
                 } else {  // central states :533-572
           T U2[NV];
-          const T roLs = (FAST && sizeof(T) == 8) ? roL * rsL : sqrt(roL);
-          const T roRs = (FAST && sizeof(T) == 8) ? roR * rsR : sqrt(roR);
+          const T roLs = (FAST && sizeof(T) == 8) ? roL * rsL : sqrt_x<T, FAST>(roL);
+          const T roRs = (FAST && sizeof(T) == 8) ? roR * rsR : sqrt_x<T, FAST>(roR);
           f1 = rcp_<T, FAST>(roLs + roRs);
           f2 = (TAPE == tape::kNone) ? fsign(T(1), Uh[bn]) : (bneg ? T(-1) : T(1));
           const T at1 = f1 * (roLs * vt1L + roRs * vt1R + (UR1[bt1] - UL1[bt1]) * f2);

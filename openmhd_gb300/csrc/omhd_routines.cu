@@ -19,6 +19,41 @@ constexpr int TPB = 256;
 __device__ __forceinline__ int lo_of(int n) { return (n < 2 ? n : 2) - 1; }
 __device__ __forceinline__ int hi_of(int n) { return (n - 1 > 1 ? n - 1 : 1) - 1; }
 
+// t = q0 + n0 (q1 + n1 q2); in 32-bit divisions where they hold t (a 64-bit one is
+// ~100 instructions)
+struct Split2 {
+  int q0, q1, q2;
+};
+__device__ __forceinline__ Split2 split2(long long t, int n0, int n1) {
+  if (t <= 0xffffffffLL) {
+    const unsigned u = (unsigned)t, l = u / (unsigned)n0;
+    return {(int)(u - l * (unsigned)n0), (int)(l % (unsigned)n1), (int)(l / (unsigned)n1)};
+  }
+  const long long l = t / n0;
+  return {(int)(t % n0), (int)(l % n1), (int)(l / n1)};
+}
+
+// reconstruct<double> with the signs and minima of minmod and MC on the integer
+// pipes (reconstruct_fp64_g: the same bits; 4-5 FP64 operations instead of ~15),
+// where no slope is infinite, NaN or so small that halving it rounds
+__device__ __forceinline__ void reconstruct_exact(int type, double wm, double w0, double wp, double& left,
+                                                  double& right) {
+  auto fine = [](double x) {
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return (h | (unsigned)__double2loint(x)) == 0u || (h >= 0x00300000u && h < 0x7ff00000u);
+  };
+  const double gA = w0 - wm, gB = wp - w0;
+  if (type == LM_MINMOD && fine(gA) && fine(gB)) {
+    reconstruct_fp64_g(LM_MINMOD, gA, gB, wm, w0, wp, left, right);
+    return;
+  }
+  if (type == LM_MC && fine(gA) && fine(gB) && fine(wp - wm)) {
+    reconstruct_fp64_g(LM_MC, gA, gB, wm, w0, wp, left, right);
+    return;
+  }
+  reconstruct<double>(type, wm, w0, wp, left, right);
+}
+
 // ---------------- u2v (2D_basic/u2v.f90:20-31) ----------------
 __global__ void k_u2v(const double* __restrict__ U, double* __restrict__ V, size_t n, double f1,
                       DevError* err) {
@@ -26,7 +61,8 @@ __global__ void k_u2v(const double* __restrict__ U, double* __restrict__ V, size
   if (c >= n) return;
   const double ro = U[RO * n + c];
   const double mx = U[MX * n + c], my = U[MY * n + c], mz = U[MZ * n + c];
-  const double vx = mx / ro, vy = my / ro, vz = mz / ro;
+  const Divisor dr = divisor(ro);
+  const double vx = div_rn(mx, dr), vy = div_rn(my, dr), vz = div_rn(mz, dr);
   const double rv2 = vx * mx + vy * my + vz * mz;
   const double bx = U[BX * n + c], by = U[BY * n + c], bz = U[BZ * n + c];
   const double B2 = bx * bx + by * by + bz * bz;
@@ -53,10 +89,8 @@ __global__ void k_limiter(const double* __restrict__ wk, double* __restrict__ wL
   const long long total = (long long)nd * n1 * n2;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
-  const int m = (int)(t % nd);
-  const long long line = t / nd;
-  const int q1 = lo1 + (int)(line % n1);
-  const int q2 = lo2 + (int)(line / n1);
+  const Split2 sp = split2(t, nd, n1);
+  const int m = sp.q0, q1 = lo1 + sp.q1, q2 = lo2 + sp.q2;
   const size_t base = (size_t)q1 * stride[a1] + (size_t)q2 * stride[a2];
   const size_t s = stride[d];
   if (type == LM_FLAT) {  // :54-71
@@ -72,7 +106,7 @@ __global__ void k_limiter(const double* __restrict__ wk, double* __restrict__ wL
     wR[base + (nd - 2) * s] = wk[base + (nd - 1) * s];  // :103
   } else {
     double l, r;
-    reconstruct<double>(type, wk[base + (m - 1) * s], wk[base + m * s], wk[base + (m + 1) * s], l, r);
+    reconstruct_exact(type, wk[base + (m - 1) * s], wk[base + m * s], wk[base + (m + 1) * s], l, r);
     wR[base + (m - 1) * s] = r;
     wL[base + m * s] = l;
   }
@@ -86,9 +120,8 @@ __global__ void k_flux(double* __restrict__ F, const double* __restrict__ VL, co
   const long long total = (long long)ni * nj * nk;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
-  const int i = is + (int)(t % ni);
-  const int j = js + (int)((t / ni) % nj);
-  const int k = ks + (int)(t / ((long long)ni * nj));
+  const Split2 sp = split2(t, ni, nj);
+  const int i = is + sp.q0, j = js + sp.q1, k = ks + sp.q2;
   const size_t n = (size_t)ix * jx * kx;
   const size_t c = (size_t)i + (size_t)ix * ((size_t)j + (size_t)jx * k);
   double L[NV], R[NV], Fo[NV];
@@ -126,12 +159,10 @@ __global__ void k_rk(int mode, double* __restrict__ U, double* __restrict__ U1, 
   const int ni = ix - 2, nj = jx - 2, nk = (nd == 3) ? kx - 2 : 1;
   const long long per = (long long)ni * nj * nk;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= per * NV) return;
-  const int m = (int)(t / per);
-  const long long r = t % per;
-  const int i = 1 + (int)(r % ni);
-  const int j = 1 + (int)((r / ni) % nj);
-  const int k = (nd == 3 ? 1 : 0) + (int)(r / ((long long)ni * nj));
+  if (t >= per) return;
+  const int m = blockIdx.y;
+  const Split2 sp = split2(t, ni, nj);
+  const int i = 1 + sp.q0, j = 1 + sp.q1, k = (nd == 3 ? 1 : 0) + sp.q2;
   const size_t n = (size_t)ix * jx * kx;
   const size_t sy = ix, sz = (size_t)ix * jx;
   const size_t q = (size_t)m * n + (size_t)i + sy * j + sz * k;
@@ -196,9 +227,8 @@ __global__ void k_set_dt(const double* __restrict__ U, const double* __restrict_
   double v = 0.0;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
-    const int i = is + (int)(t % ni);
-    const int j = js + (int)((t / ni) % nj);
-    const int k = ks + (int)(t / ((long long)ni * nj));
+    const Split2 sp = split2(t, ni, nj);
+    const int i = is + sp.q0, j = js + sp.q1, k = ks + sp.q2;
     const size_t c = (size_t)i + (size_t)ix * ((size_t)j + (size_t)jx * k);
     v = fmax2(cell_speed(U, V, n, c, nd, gamma), v);
   }
@@ -469,7 +499,7 @@ int do_rk(int mode, double* U, double* U1, const double* F, const double* G, con
   const double dtx = (mode == 2) ? 0.5 * dt / dx : dt / dx;  // rk.f90:22, :76
   const long long per = (long long)(ix - 2) * (jx - 2) * (nd == 3 ? kx - 2 : 1);
   if (per > 0)
-    k_rk<<<ceil_div(per * NV, TPB), TPB, 0, lib_stream()>>>(mode, Ud, U1d, Fd, Gd, Hd, dtx, ix, jx, kx, nd);
+    k_rk<<<dim3(ceil_div(per, TPB), NV), TPB, 0, lib_stream()>>>(mode, Ud, U1d, Fd, Gd, Hd, dtx, ix, jx, kx, nd);
   return a.finish();
 }
 

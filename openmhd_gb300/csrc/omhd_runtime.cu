@@ -189,8 +189,8 @@ __global__ void k_fastmath_probe(const double* __restrict__ x, long long n, doub
   }
 }
 
-// mul_int(a, b), whether it refuses the operands (1.0) and half_exact(a): three
-// planes of n values
+// mul_int(a, b), whether it refuses the operands (1.0), half_exact(a),
+// div_rn(a, b) and sqrt_rn(a): five planes of n values
 __global__ void k_mul_probe(const double* __restrict__ a, const double* __restrict__ b, long long n,
                             double* __restrict__ out) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -198,6 +198,8 @@ __global__ void k_mul_probe(const double* __restrict__ a, const double* __restri
     out[i] = mul_int(a[i], b[i], bad);
     out[n + i] = bad ? 1.0 : 0.0;
     out[2 * n + i] = half_exact(a[i]);
+    out[3 * n + i] = div_rn(a[i], b[i]);
+    out[4 * n + i] = sqrt_rn(a[i]);
   }
 }
 

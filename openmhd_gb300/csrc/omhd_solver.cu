@@ -173,7 +173,8 @@ __device__ __forceinline__ double cell_cfl_speed(const double (&u)[NV], double g
   const double f1g = gamma - 1;
   const double ro = u[RO];
   const double mx = u[MX], my = u[MY], mz = u[MZ];
-  const double vx = mx / ro, vy = my / ro, vz = mz / ro;
+  const Divisor dr = divisor(ro);
+  const double vx = div_rn(mx, dr), vy = div_rn(my, dr), vz = div_rn(mz, dr);
   const double rv2 = vx * mx + vy * my + vz * mz;
   const double bx = u[BX], by = u[BY], bz = u[BZ];
   const double B2 = bx * bx + by * by + bz * bz;

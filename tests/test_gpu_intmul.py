@@ -1,6 +1,6 @@
-"""The FP64 products that the performance kernels make on the integer pipes
-(mul_int, half_exact in openmhd_gb300/csrc/omhd_fastmath.h): against IEEE
-products on the host, and whole steps in units that reach the ends of their
+"""The FP64 products, quotients and roots that the kernels make on the integer pipes
+(mul_int, half_exact, div_rn, sqrt_rn in openmhd_gb300/csrc/omhd_fastmath.h):
+against IEEE results on the host, and whole steps in units that reach the ends of their
 range, where a face is solved with FP64-pipe products instead."""
 import ctypes as C
 import dataclasses
@@ -19,10 +19,10 @@ def _probe(lib, a, b):
     import torch
 
     at, bt = (torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (a, b))
-    out = torch.empty(3 * len(a), dtype=torch.float64, device="cuda")
+    out = torch.empty(5 * len(a), dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
     assert lib.omhd_probe_mul(C.c_void_p(at.data_ptr()), C.c_void_p(bt.data_ptr()), len(a), C.c_void_p(out.data_ptr())) == 0
-    return out.cpu().numpy().reshape(3, -1)
+    return out.cpu().numpy().reshape(5, -1)
 
 
 def _significands(rng, n):
@@ -44,7 +44,7 @@ def test_products_equal_ieee(cuda_lib, lo, hi):
     for v in ab:
         v[rng.integers(0, n, n // 50)] = rng.choice([0.0, -0.0], n // 50)
     a, b = ab
-    got, bad, half = _probe(cuda_lib, a, b)
+    got, bad, half, _, _ = _probe(cuda_lib, a, b)
     with np.errstate(under="ignore"):
         want, whalf = a * b, a * 0.5
     assert not bad.any()
@@ -82,10 +82,33 @@ def test_operands_out_of_range_are_refused(cuda_lib):
     a = np.array([x for x in big for _ in range(4)] + [2.0**511 - 2.0**458])
     b = np.array([1.0, 0.0, 1e-300, 5e-324] * len(big) + [1.0])
     for u, v in ((a, b), (b, a)):
-        _, bad, _ = _probe(cuda_lib, u, v)
+        bad = _probe(cuda_lib, u, v)[1]
         assert bad[:-1].all() and not bad[-1]
     half = _probe(cuda_lib, np.array([np.inf, -np.inf, np.nan]), np.ones(3))[2]
     assert half[0] == np.inf and half[1] == -np.inf and np.isnan(half[2])
+
+
+@pytest.mark.parametrize("lo,hi", [(-60, 60), (-1, 1), (-1022, 1023)])
+def test_quotients_and_roots_equal_ieee(cuda_lib, lo, hi):
+    """Correctly rounded, bit for bit, on exact quotients and squares, their
+    neighbours, zeros, subnormals, infinities and NaN."""
+    rng = np.random.default_rng(hi)
+    n = 1 << 21
+    a, b = (np.ldexp(1 + _significands(rng, n) * 2.0**-52, rng.integers(lo, hi + 1, n)) * rng.choice([-1.0, 1.0], n)
+            for _ in range(2))
+    k = n // 8
+    with np.errstate(all="ignore"):
+        a[:k] = a[:k] * b[:k]  # near an exact quotient
+        a[k : 2 * k] = b[k : 2 * k] ** 2  # near an exact root
+        a[2 * k : 3 * k] = np.nextafter(b[2 * k : 3 * k] ** 2, rng.choice([0, np.inf], k))
+        special = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, -1e-310, TINY, 1.7e308, 1.0])
+        for v in (a, b):
+            v[rng.integers(0, n, n // 100)] = rng.choice(special, n // 100)
+        _, _, _, div, root = _probe(cuda_lib, a, b)
+        for got, want in ((div, a / b), (root, np.sqrt(a))):
+            nan = np.isnan(want)
+            assert np.array_equal(np.isnan(got), nan)
+            assert np.array_equal(got[~nan].view(np.int64), want[~nan].view(np.int64))
 
 
 @pytest.mark.parametrize("ro,pr", [(1.0, 1.0), (1e155, 1e150), (1e-150, 1e-150), (1e-3, 1e149)])
