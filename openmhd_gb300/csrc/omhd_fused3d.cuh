@@ -220,7 +220,7 @@ __device__ __forceinline__ void load_plane(const StageArgs& a, T* W, int slot, i
     if (a.stage == 1) ps = glmf * ps;
     T w[NV];
     double pr, ro;
-    u2v_cell<T, OMHD_FAST>(u, f1g, f1g32, ps, w, pr, ro);  // 3D_basic/u2v.f90
+    u2v_cell<T, OMHD_FAST, OMHD_FAST && sizeof(T) == 8>(u, f1g, f1g32, ps, w, pr, ro);  // 3D_basic/u2v.f90
 #pragma unroll
     for (int v = 0; v < NV; ++v) Ws[v * PL + q] = w[v];
     if (own_plane && cx_in && cy_in && gi <= ix - 2 && gj <= jx - 2) {  // u2v.f90:36-45, owner check

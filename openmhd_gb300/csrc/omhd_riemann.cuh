@@ -890,7 +890,10 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
 // difference of energies -- amplifies the rounding of its inputs at most
 // ~4-fold; FP64 recovery, then rounding, everywhere else (low beta, high
 // Mach, and every unphysical state, whose check then sees FP64 values).
-template <class T, bool FAST>
+// INTMUL: the FP64 recovery's products on the integer pipes (not in the mixed 3D
+// kernel, whose FP64 pipe has room: 14.97 against 14.78 ms on Harris 256x128x256;
+// the 2D ensemble's 16.0 -> 15.5 ms).
+template <class T, bool FAST, bool INTMUL = FAST>
 __device__ __forceinline__ void u2v_cell(const double (&u)[NV], double f1g, float f1g32, double psi, T (&w)[NV],
                                          double& pr, double& ro) {
   if constexpr (sizeof(T) == 4) {
@@ -920,12 +923,12 @@ __device__ __forceinline__ void u2v_cell(const double (&u)[NV], double f1g, floa
   const double bx = u[BX], by = u[BY], bz = u[BZ];
   const double ir = rcp_<double, FAST>(r);  // one reciprocal for the three velocities
   double vx, vy, vz, p;
-  if constexpr (FAST && sizeof(T) == 8) {  // the plain products on the integer pipes, as in the Riemann solver
+  if constexpr (INTMUL) {  // the plain products on the integer pipes, as in the Riemann solver
     auto recover = [&](auto& mul) {
       vx = mul(mx, ir);
       vy = mul(my, ir);
       vz = mul(mz, ir);
-      const double e2 = fma(vz, mz, fma(vy, my, mul(vx, mx))) + fma(bz, bz, fma(by, by, mul(bx, bx)));
+      const double e2 = fma(vz, mz, fma(vx, mx, mul(vy, my))) + fma(bz, bz, fma(bx, bx, mul(by, by)));
       p = mul(f1g, fma(-0.5, e2, u[EN]));
     };
     MulInt mi;
