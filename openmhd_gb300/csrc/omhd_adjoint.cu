@@ -236,6 +236,29 @@ __global__ void __launch_bounds__(128) k_adj_faces(AdjGeo g, const double* __res
   }
 }
 
+// Derivative of a cell's limited slope with respect to the cell itself (d = 0) or to
+// its lower / upper neighbour (d = -1 / +1), for the recorded selection: the face
+// states are w0 +- slope, so the neighbour's gradient takes the weight times
+// (gUp - gLo), the cell's own (1 + weight) gUp + (1 - weight) gLo.  A selected
+// constant instead of selected sums (recon_vjp_code): a predicated-off FP64
+// instruction holds the FP64 pipe, and the kernel was bound by it (98 us for
+// 512x256; 14 of its operations per variable, direction and cell, now 6).
+template <int d>
+__device__ __forceinline__ double recon_weight(int lm, unsigned char code) {
+  const int sel = code & 3;
+  const unsigned one = lm == LM_MC ? 0x3ff00000u : 0x3fe00000u;  // 1 or 1/2 (high word)
+  unsigned h = 0u;
+  if (d == 0) {
+    h = sel == tape::kLimA ? one : (sel == tape::kLimB ? one | 0x80000000u : 0u);
+  } else {
+    const unsigned q = one - 0x00200000u;  // a quarter of it: MC's central slope, with its sign
+    const unsigned c = (code & tape::kLimCNeg) ? q | 0x80000000u : q;
+    h = sel == tape::kLimC ? c : (sel == (d < 0 ? tape::kLimA : tape::kLimB) ? one : 0u);
+    if (d < 0 && h) h ^= 0x80000000u;
+  }
+  return __hiloint2double((int)h, 0);
+}
+
 // Per cell: adjoint of the (up to) three reconstructions per direction that
 // read the cell, then of u2v; adds a1*A + B on the interior (the RK
 // pass-through terms) and the GLM factor on psi when asked.
@@ -268,11 +291,15 @@ __global__ void __launch_bounds__(256) k_adj_cells(AdjGeo g, const double* __res
       const size_t cm = (d == -1) ? c + s : ((d == 1) ? c - s : c);
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        double gm = 0.0, g0 = 0.0, gp = 0.0;
         const unsigned char k = tlim ? tlim[(A * NV + v) * n + cm]
                                      : adj::recon_code(g.lm, W[v * n + cm - s], W[v * n + cm], W[v * n + cm + s]);
-        adj::recon_vjp_code(g.lm, k, gUp[(A * NV + v) * n + cm], gLo[(A * NV + v) * n + cm], gm, g0, gp);
-        gw[v] += (d == -1) ? gm : ((d == 0) ? g0 : gp);
+        const double gl = gUp[(A * NV + v) * n + cm], gr = gLo[(A * NV + v) * n + cm];
+        if (d == 0) {
+          const double q = recon_weight<0>(g.lm, k);
+          gw[v] = fma(1.0 - q, gr, fma(1.0 + q, gl, gw[v]));
+        } else {
+          gw[v] = fma(d < 0 ? recon_weight<-1>(g.lm, k) : recon_weight<1>(g.lm, k), gl - gr, gw[v]);
+        }
       }
     }
   }
