@@ -226,11 +226,11 @@ int omhd_probe_fp32_peak(double* gflops);
  * (the second and last by the device's IEEE division and square root);
  * synchronous, on the default stream */
 int omhd_probe_fastmath(const double* x_dev, long long n, double* out_dev);
-/* probe of the integer-pipe FP64 products, quotients and roots of the kernels (no
- * counterpart in the reference): for n device doubles a and b, writes 5*n
+/* probe of the integer-pipe FP64 products, quotients, roots and differences of the
+ * kernels (no counterpart in the reference): for n device doubles a and b, writes 6*n
  * device doubles to out, planes mul_int(a, b), 1.0 where it refuses the operands
  * (its value is then meaningless) else 0.0, half_exact(a), div_rn(a, b),
- * sqrt_rn(a); synchronous, on the default stream */
+ * sqrt_rn(a), sub_f32((float)a, (float)b); synchronous, on the default stream */
 int omhd_probe_mul(const double* a_dev, const double* b_dev, long long n, double* out_dev);
 /* probe of the integer-pipe binary32 <-> binary64 conversions of the
  * FP32-mixed kernels (no counterpart in the reference): for n device values,

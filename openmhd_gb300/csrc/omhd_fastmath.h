@@ -274,6 +274,39 @@ __device__ __forceinline__ double widen_f32(float f) {
   return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
 }
 
+// widen_f32(a) - widen_f32(b), rounded to binary64, without the FP64 pipe (the same
+// bits for all arguments; a NaN stays one).  s = a - b in
+// binary32 and its exact error e (Knuth's two-sum) add up to a - b; s's binary64
+// bits and e in units of s's last binary64 place are then added as integers, which
+// cannot carry out of s's binade but where s is a power of two and e points to the
+// binade below, whose places are half as wide.  e in those units has to be rounded
+// to an integer only if it reaches below 53 bits, and to even as the sum's own parity
+// is e's (s ends in 29 zeros).  Two operands below 2^-30 are scaled by 2^96 so that s
+// and e stay normal, others by 2^-2 so that s stays finite.  ~33 instructions; the FP64 subtraction holds the SM's FP64 pipe
+// for 19 cycles, in which its four schedulers issue 76.
+__device__ __forceinline__ float mul_ftz(float x, float y) {  // subnormals are zeros
+  float r;
+  asm("mul.rn.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ double sub_f32(float a, float b) {
+  const bool small = fmaxf(fabsf(a), fabsf(b)) < 0x1p-30f;
+  const float scale = small ? 0x1p96f : 0x1p-2f;
+  a = mul_ftz(a, scale);
+  b = mul_ftz(b, scale);
+  const float s = __fsub_rn(a, b), t = __fsub_rn(s, a);
+  const float e = __fsub_rn(__fsub_rn(a, __fsub_rn(s, t)), __fadd_rn(b, t));
+  const unsigned u = __float_as_uint(s), mag = u & 0x7fffffffu;
+  // +-2^(1-Es), the sign that of s; 0 for infinity and NaN
+  const float x = __fmul_rn(e, __uint_as_float((0x7f800000u - (u & 0x7f800000u)) | (u & 0x80000000u)));
+  const bool below = (u << 9) == 0u && x < 0.0f;
+  const int j = __float2int_rn(__fmul_rn(x, below ? 0x1p52f : 0x1p51f));  // 0 for NaN
+  const unsigned hi = (mag >> 3) + (mag >= 0x7f800000u ? 0x70000000u : small ? 0x32000000u : 0x38200000u);
+  unsigned long long r = (((unsigned long long)hi << 32) | (u << 29)) + (unsigned long long)(long long)j;
+  r = mag == 0u ? 0ull : r;
+  return __hiloint2double((int)((unsigned)(r >> 32) | (u & 0x80000000u)), (int)(unsigned)r);
+}
+
 __device__ __forceinline__ float narrow_f64(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const unsigned ahi = hi & 0x7fffffffu;

@@ -50,13 +50,11 @@ struct Geo2 {
   static constexpr int NXFP = round32(NXF);       // x faces padded to whole warps
   // one thread per y face (or padded x face), at least one per cell
   static constexpr int NT = imax(imax(NXFP, round32(NYF)), round32(TX * TY));
-  // face states in T, face fluxes in FP64 (the flux differences are FP64,
-  // so each flux is widened once, when it is stored)
+  // primitives and face states; a face's flux replaces one of its states
   template <class T>
   static constexpr size_t smem_bytes() {
-    return sizeof(T) * (size_t)NV * (RY * RX + 2 * (NXS + NYS)) + sizeof(double) * (size_t)NV * (NXF + NYF);
+    return sizeof(T) * (size_t)NV * (RY * RX + 2 * (NXS + NYS));
   }
-  static_assert((NV * (RY * RX + 2 * (NXS + NYS))) % 2 == 0, "flux block must start 8-byte aligned");
 };
 // tile of the single-grid stage kernel per arithmetic type.  FP64: 16x16, whose
 // halo is the smallest of the shapes a 288-thread CTA serves (1.5 loaded cells
@@ -161,7 +159,7 @@ struct TileMem {
   const T* Bf;
   T* bcopy;
   T *SLx, *SRx, *SLy, *SRy;
-  double *FX, *FY;
+  T *FX, *FY;
   int fxv, fxr, fyv;
 };
 
@@ -214,11 +212,11 @@ __device__ __forceinline__ TileMem<T> tile_mem_separate(unsigned char* smem_raw)
   m.SRx = m.SLx + NV * G::NXS;
   m.SLy = m.SRx + NV * G::NXS;
   m.SRy = m.SLy + NV * G::NYS;
-  m.FX = reinterpret_cast<double*>(m.SRy + NV * G::NYS);
-  m.FY = m.FX + NV * G::NXF;
-  m.fxv = G::NXF;
-  m.fxr = G::TX + 1;
-  m.fyv = G::NYF;
+  m.FX = m.SLx;  // flux of x face (fx, cy) in the SLx slot of cell fx of row cy
+  m.fxv = G::NXS;
+  m.fxr = G::TX + 2;
+  m.FY = m.SLy;  // flux of y face (cx, fy) in the SLy slot of cell fy of column cx
+  m.fyv = G::NYS;
   return m;
 }
 
@@ -624,7 +622,7 @@ __device__ __forceinline__ void phase_flux(const StageArgs& a, int bxi, int byi,
         }
       }
 #pragma unroll
-      for (int v = 0; v < NV; ++v) m.FX[v * m.fxv + cy * m.fxr + fx] = to_f64<T>(Fo[v]);
+      for (int v = 0; v < NV; ++v) m.FX[v * m.fxv + cy * m.fxr + fx] = Fo[v];
     } else {
       const int qq = q - NXFP;
       const int cx = qq % TX, fy = qq / TX;
@@ -659,7 +657,7 @@ __device__ __forceinline__ void phase_flux(const StageArgs& a, int bxi, int byi,
         }
       }
 #pragma unroll
-      for (int v = 0; v < NV; ++v) m.FY[v * m.fyv + fy * TX + cx] = to_f64<T>(Fo[v]);
+      for (int v = 0; v < NV; ++v) m.FY[v * m.fyv + fy * TX + cx] = Fo[v];
     }
   }
 }
@@ -702,12 +700,20 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
     // the variables, in blocks too long to be predicated: a predicated-off FP64
     // instruction holds the FP64 pipe like any other, and with the choices inside
     // the ensemble kernel spent half of its FP64 time on the results not taken.
+    // Mixed: the differences of binary32 fluxes and the halving are made on the FP32
+    // and integer pipes (sub_f32, half_exact: the same bits), 18 of the 54 FP64
+    // operations of a cell in stage 1 and 27 of 74 in stage 2; KH 2048x1024: 338 to
+    // 299 and 452 to 378 us, the FP64 pipe 55 to 42 % busy, issue slots 50 to 60 %.
     auto dF = [&](int v) {  // F(i-1/2) - F(i+1/2) in FP64
-      const double* fx = m.FX + v * m.fxv + ty * m.fxr + tx;
-      return fx[0] - fx[1];
+      const T* fx = m.FX + v * m.fxv + ty * m.fxr + tx;
+      return sub_f64<T>(fx[0], fx[1]);
     };
-    auto gm = [&](int v) { return m.FY[v * m.fyv + ty * TX + tx]; };
-    auto gp = [&](int v) { return m.FY[v * m.fyv + (ty + 1) * TX + tx]; };
+    auto gm = [&](int v) { return to_f64<T>(m.FY[v * m.fyv + ty * TX + tx]); };
+    auto gp = [&](int v) { return to_f64<T>(m.FY[v * m.fyv + (ty + 1) * TX + tx]); };
+    auto dG = [&](int v) {
+      const T* fy = m.FY + v * m.fyv + ty * TX + tx;
+      return sub_f64<T>(fy[0], fy[TX]);
+    };
     double u0[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) u0[v] = Ubase[v * N + c];
@@ -717,11 +723,11 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
       // operations a variable instead of 5 or 8, as many roundings of the sum
       if (rk2) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) out[v] = fma(dtx, fma(ryx, gm(v) - gp(v), dF(v)), ub(v));
+        for (int v = 0; v < NV; ++v) out[v] = fma(dtx, fma(ryx, dG(v), dF(v)), ub(v));
       } else {
 #pragma unroll
         for (int v = 0; v < NV; ++v)
-          out[v] = half_exact(fma(dtx, fma(ryx, gm(v) - gp(v), dF(v)), ub(v) + U1[v * N + c]));
+          out[v] = half_exact(fma(dtx, fma(ryx, dG(v), dF(v)), ub(v) + U1[v * N + c]));
       }
     } else {
       double d[NV];
@@ -730,14 +736,14 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
         for (int v = 0; v < NV; ++v) d[v] = dtx * (dF(v) + gm(v) - gp(v));  // rk.f90:26-35 operation order
       } else {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) d[v] = dtx * dF(v) + dty * (gm(v) - gp(v));
+        for (int v = 0; v < NV; ++v) d[v] = dtx * dF(v) + dty * dG(v);
       }
       if (rk2) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) out[v] = ub(v) + d[v];  // rk_tvd21 / rk_std21 / rk_std22
       } else {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) out[v] = 0.5 * (ub(v) + U1[v * N + c] + d[v]);  // rk_tvd22 (rk.f90:56-66)
+        for (int v = 0; v < NV; ++v) out[v] = half_<OMHD_FAST>(ub(v) + U1[v * N + c] + d[v]);  // rk_tvd22 (rk.f90:56-66)
       }
     }
     if (stage2) out[PS] = glmf * out[PS];  // second GLM half (main.f90:185)

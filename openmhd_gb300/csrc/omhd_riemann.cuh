@@ -122,6 +122,19 @@ __device__ __forceinline__ double to_f64(T x) {
   else
     return x;
 }
+// a - b in FP64
+template <class T>
+__device__ __forceinline__ double sub_f64(T a, T b) {
+  if constexpr (sizeof(T) == 4)
+    return sub_f32(a, b);
+  else
+    return a - b;
+}
+// x / 2, by the exponent in the FAST builds
+template <bool FAST>
+__device__ __forceinline__ double half_(double x) {
+  return FAST ? half_exact(x) : 0.5 * x;
+}
 
 enum { LM_FLAT = 0, LM_MINMOD = 1, LM_MC = 2, LM_VANLEER = 3, LM_KOREN = 4 };
 enum { FX_LLF = 0, FX_HLL = 1, FX_HLLC = 2, FX_HLLD = 3, FX_LHLLD = 4 };

@@ -190,7 +190,8 @@ __global__ void k_fastmath_probe(const double* __restrict__ x, long long n, doub
 }
 
 // mul_int(a, b), whether it refuses the operands (1.0), half_exact(a),
-// div_rn(a, b) and sqrt_rn(a): five planes of n values
+// div_rn(a, b), sqrt_rn(a) and sub_f32 of a and b as binary32 numbers: six planes of
+// n values
 __global__ void k_mul_probe(const double* __restrict__ a, const double* __restrict__ b, long long n,
                             double* __restrict__ out) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -200,6 +201,7 @@ __global__ void k_mul_probe(const double* __restrict__ a, const double* __restri
     out[2 * n + i] = half_exact(a[i]);
     out[3 * n + i] = div_rn(a[i], b[i]);
     out[4 * n + i] = sqrt_rn(a[i]);
+    out[5 * n + i] = sub_f32((float)a[i], (float)b[i]);
   }
 }
 

@@ -1,5 +1,5 @@
-"""The FP64 products, quotients and roots that the kernels make on the integer pipes
-(mul_int, half_exact, div_rn, sqrt_rn in openmhd_gb300/csrc/omhd_fastmath.h):
+"""The FP64 products, quotients, roots and differences that the kernels make on the integer pipes
+(mul_int, half_exact, div_rn, sqrt_rn, sub_f32 in openmhd_gb300/csrc/omhd_fastmath.h):
 against IEEE results on the host, and whole steps in units that reach the ends of their
 range, where a face is solved with FP64-pipe products instead."""
 import ctypes as C
@@ -19,10 +19,10 @@ def _probe(lib, a, b):
     import torch
 
     at, bt = (torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (a, b))
-    out = torch.empty(5 * len(a), dtype=torch.float64, device="cuda")
+    out = torch.empty(6 * len(a), dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
     assert lib.omhd_probe_mul(C.c_void_p(at.data_ptr()), C.c_void_p(bt.data_ptr()), len(a), C.c_void_p(out.data_ptr())) == 0
-    return out.cpu().numpy().reshape(5, -1)
+    return out.cpu().numpy().reshape(6, -1)
 
 
 def _significands(rng, n):
@@ -44,7 +44,7 @@ def test_products_equal_ieee(cuda_lib, lo, hi):
     for v in ab:
         v[rng.integers(0, n, n // 50)] = rng.choice([0.0, -0.0], n // 50)
     a, b = ab
-    got, bad, half, _, _ = _probe(cuda_lib, a, b)
+    got, bad, half = _probe(cuda_lib, a, b)[:3]
     with np.errstate(under="ignore"):
         want, whalf = a * b, a * 0.5
     assert not bad.any()
@@ -88,6 +88,32 @@ def test_operands_out_of_range_are_refused(cuda_lib):
     assert half[0] == np.inf and half[1] == -np.inf and np.isnan(half[2])
 
 
+@pytest.mark.parametrize("lo,hi,gap", [(-3, 3, 3), (-125, 128, 40), (-125, -88, 60), (100, 128, 120)])
+def test_differences_of_binary32_equal_ieee(cuda_lib, lo, hi, gap):
+    """sub_f32: the binary64 difference of two binary32 numbers, bit for bit, over
+    operand pairs that cancel, that fill 53 bits and that exceed them, next to
+    powers of two, and zeros, infinities and NaN."""
+    rng = np.random.default_rng(17)
+    n = 1 << 20
+    e = rng.integers(lo, hi, n)
+    f = np.clip(e + rng.integers(-gap, gap + 1, n), -126, 127)
+    m = [(1.0 + (_significands(rng, n) >> 29) / 2.0**23) * rng.choice([-1.0, 1.0], n) for _ in range(2)]
+    m[0][: n // 4] = 1.0
+    a, b = np.ldexp(m[0], e).astype(np.float32), np.ldexp(m[1], f).astype(np.float32)
+    a[-1000:-500] = b[-1000:-500]
+    sp = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 1.0, -1.0, 2.0**-126, 3.4e38, -3.4e38], np.float32)
+    sa, sb = (v.ravel() for v in np.meshgrid(sp, sp))
+    swap = rng.random(n) < 0.5
+    a, b = np.where(swap, b, a), np.where(swap, a, b)
+    a, b = np.concatenate([a, sa]), np.concatenate([b, sb])
+    with np.errstate(invalid="ignore"):
+        want = a.astype(np.float64) - b.astype(np.float64)
+    got = _probe(cuda_lib, a.astype(np.float64), b.astype(np.float64))[5]
+    nan = np.isnan(want)
+    assert np.isnan(got[nan]).all()
+    assert np.array_equal(got[~nan].view(np.uint64), want[~nan].view(np.uint64))
+
+
 @pytest.mark.parametrize("lo,hi", [(-60, 60), (-1, 1), (-1022, 1023)])
 def test_quotients_and_roots_equal_ieee(cuda_lib, lo, hi):
     """Correctly rounded, bit for bit, on exact quotients and squares, their
@@ -104,7 +130,7 @@ def test_quotients_and_roots_equal_ieee(cuda_lib, lo, hi):
         special = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, -1e-310, TINY, 1.7e308, 1.0])
         for v in (a, b):
             v[rng.integers(0, n, n // 100)] = rng.choice(special, n // 100)
-        _, _, _, div, root = _probe(cuda_lib, a, b)
+        div, root = _probe(cuda_lib, a, b)[3:5]
         for got, want in ((div, a / b), (root, np.sqrt(a))):
             nan = np.isnan(want)
             assert np.array_equal(np.isnan(got), nan)
