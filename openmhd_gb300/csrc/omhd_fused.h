@@ -113,4 +113,12 @@ int launch_stage3d_fp64(const StageArgs& a, cudaStream_t s);
 int launch_stage3d_parity(const StageArgs& a, cudaStream_t s);
 int launch_stage3d_mixed(const StageArgs& a, cudaStream_t s);
 
+// SMs of the current device
+inline int sm_count(int* nsm) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev);
+  return (int)e;
+}
+
 }  // namespace omhd

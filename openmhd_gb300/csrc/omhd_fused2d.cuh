@@ -58,10 +58,11 @@ struct Geo2 {
 };
 // tile of the single-grid stage kernel per arithmetic type.  FP64: 16x16, whose
 // halo is the smallest of the shapes a 288-thread CTA serves (1.5 loaded cells
-// per cell).  FP32-mixed: 16x8 tiles of 160 threads, four CTAs per SM (96
-// registers): more CTAs interleave their barrier-separated phases; measured on
-// KH 4096x2048, 16x8 at 4 / 3 CTAs per SM and 16x16 / 32x8 / 64x4 at 2 CTAs per
-// SM gave 1.985e9 / 1.819e9 and 1.894e9 / 1.868e9 / 1.824e9 cell-updates/s
+// per cell).  FP32-mixed: 16x8 tiles of 160 threads, four or five CTAs per SM
+// (launch_one): more CTAs interleave their barrier-separated phases; ms a step of
+// KH 4096x2048 / Orszag-Tang 256^2: 16x8 at 5 CTAs per SM 2.86 / 0.0490 and at 4
+// 2.96 / 0.0481, 16x10 at 4 2.91 / 0.0480 (64^2 7 % slower), 16x12 at 3 2.95 /
+// 0.0524, 16x16 at 2 3.06 / 0.0492, 32x8 at 2 3.11 / 0.0523, 16x4 at 7 3.23 / 0.0473
 // (build-time constants, for tuning)
 #ifndef OMHD_MIXED_TILE_X
 #define OMHD_MIXED_TILE_X 16
@@ -812,9 +813,8 @@ __device__ __forceinline__ double stage2d_tile(const StageArgs& a, int bxi, int 
 }
 
 // one CTA per tile of one grid
-template <class T, int FLUX, int TAPE = tape::kNone>
-__global__ void __launch_bounds__(GeoFor<T>::type::NT, sizeof(T) == 4 ? OMHD_MIXED_MIN_CTAS : 1)
-    k_stage2d(const StageArgs a) {
+template <class T, int FLUX, int TAPE = tape::kNone, int CTAS = sizeof(T) == 4 ? OMHD_MIXED_MIN_CTAS : 1>
+__global__ void __launch_bounds__(GeoFor<T>::type::NT, CTAS) k_stage2d(const StageArgs a) {
   using G = typename GeoFor<T>::type;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red32[32];
@@ -1051,10 +1051,9 @@ int launch_pipe(const StageArgs& a, cudaStream_t s) {
   static std::atomic<unsigned long long> configured{0};
   int r = set_smem_attr_once(k_stage2d_pipe<FLUX, TAPE, NPW>, bytes, configured);
   if (r) return r;
-  int dev = 0, nsm = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return (int)e;
+  int nsm = 0;
+  r = sm_count(&nsm);
+  if (r) return r;
   const int ntx = (a.ix - 2 + PipeGeo::TX - 1) / PipeGeo::TX;
   const int ty = pick_rows(ntx, a.jx - 2, nsm);
   const int ntiles = ntx * ((a.jx - 2 + ty - 1) / ty);
@@ -1146,16 +1145,38 @@ __global__ void __launch_bounds__(G::NT, sizeof(T) == 4 ? (G::NT <= 160 ? 4 : 2)
   }
 }
 
-template <class T, int FLUX, int TAPE = tape::kNone>
-int launch_one(const StageArgs& a, cudaStream_t s) {
+template <class T, int FLUX, int TAPE, int CTAS>
+int launch_ctas(const StageArgs& a, dim3 grid, cudaStream_t s) {
   using G = typename GeoFor<T>::type;
   const size_t bytes = G::template smem_bytes<T>();
   static std::atomic<unsigned long long> configured{0};
-  const int r = set_smem_attr_once(k_stage2d<T, FLUX, TAPE>, bytes, configured);
+  const int r = set_smem_attr_once(k_stage2d<T, FLUX, TAPE, CTAS>, bytes, configured);
   if (r) return r;
-  dim3 grid((a.ix - 2 + G::TX - 1) / G::TX, (a.jx - 2 + G::TY - 1) / G::TY);
-  k_stage2d<T, FLUX, TAPE><<<grid, G::NT, bytes, s>>>(a);
+  k_stage2d<T, FLUX, TAPE, CTAS><<<grid, G::NT, bytes, s>>>(a);
   return (int)cudaGetLastError();
+}
+
+// FP32-mixed HLLD in two builds: 96 registers and four CTAs per SM, or 72 (120 bytes
+// spilled) and five, whose phases cover each other better once the tiles fill more
+// than one round of four.  ms a step with four / five: 64^2 0.0295 / 0.0299, 256^2
+// (512 tiles on 152 SMs) 0.0481 / 0.0490, 700^2 0.2080 / 0.2063, 1000x500 0.2129 /
+// 0.2027, 2048x1024 0.784 / 0.749, 4096x2048 2.960 / 2.855.
+template <class T, int FLUX, int TAPE = tape::kNone>
+int launch_one(const StageArgs& a, cudaStream_t s) {
+  using G = typename GeoFor<T>::type;
+  dim3 grid((a.ix - 2 + G::TX - 1) / G::TX, (a.jx - 2 + G::TY - 1) / G::TY);
+  if constexpr (sizeof(T) == 4) {
+    if constexpr (FLUX == FX_HLLD && TAPE == tape::kNone) {
+      int nsm = 0;
+      const int r = sm_count(&nsm);
+      if (r) return r;
+      if ((long long)grid.x * grid.y > (long long)OMHD_MIXED_MIN_CTAS * nsm)
+        return launch_ctas<T, FLUX, TAPE, OMHD_MIXED_MIN_CTAS + 1>(a, grid, s);
+    }
+    return launch_ctas<T, FLUX, TAPE, OMHD_MIXED_MIN_CTAS>(a, grid, s);
+  } else {
+    return launch_ctas<T, FLUX, TAPE, 1>(a, grid, s);
+  }
 }
 
 template <class T, int FLUX, class G>

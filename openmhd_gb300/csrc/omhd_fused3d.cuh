@@ -791,13 +791,6 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
   }
 }
 
-inline int sm_count(int* nsm) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev);
-  return (int)e;
-}
-
 template <class G>
 inline long long columns_of(const StageArgs& a) {
   return (long long)((a.ix - 2 + G::TX - 1) / G::TX) * ((a.jx - 2 + G::TY - 1) / G::TY);
