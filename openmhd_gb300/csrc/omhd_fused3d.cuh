@@ -26,9 +26,10 @@ namespace OMHD_VARIANT {
 namespace d3 {
 
 // A column of TX x TY cells and the CTAs per SM its kernel is built for.
-template <int TX_, int TY_, int CTAS_>
+template <int TX_, int TY_, int CTAS_, int EXTRA_ = 0>
 struct Col {
-  static constexpr int TX = TX_, TY = TY_, CTAS = CTAS_, NT = TX * TY;
+  static constexpr int TX = TX_, TY = TY_, CTAS = CTAS_, CELLS = TX * TY;
+  static constexpr int NT = CELLS + 32 * EXTRA_;  // EXTRA_ warps without cells
   static_assert(TY * NV <= NT - TX, "the x and y wall fixes use disjoint threads");
   static constexpr int RX = TX + 4, RY = TY + 4, PL = RX * RY;  // plane of the halo tile
   static constexpr int XS = TX + 2, NXS3 = TY * XS;             // cells reconstructed in x (a row strip per tile row)
@@ -56,9 +57,15 @@ struct Col {
 #endif
 template <class T>
 using DefaultCol = Col<OMHD_3D_TILE_X, OMHD_3D_TILE_Y, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 1>;
-// FP64 HLLD with fused multiply-adds: 16x16, or two 16x8 CTAs per SM (pick_col)
-using WideCol = Col<16, 16, 1>;
-using SmallCol = Col<16, 8, 2>;
+// FP64 HLLD with fused multiply-adds: 16x16, or two 16x8 CTAs per SM
+// (launch_best3d), with a warp more than the cells need.  The 16x16 plane's 288
+// pairs of face states and 544 x and y faces are 9 and 17 warps' worth, which eight
+// warps did in rounds of 8 and 1: a warp alone on the SM gets a third of the FP64
+// pipe, and a quarter of a plane's time went that way (224 registers and 444 bytes
+// spilled instead of 255; Harris 256x128x256 33.3 -> 28.6 ms per step, two extra
+// warps 28.8, mixed 6.17 -> 6.75: not used there).  16x8: loop 100x100x200 5.70 -> 5.25.
+using WideCol = Col<16, 16, 1, 1>;
+using SmallCol = Col<16, 8, 2, 1>;
 constexpr int NRING = 4;
 constexpr int ZCHUNK = 64;  // most z planes marched by one CTA
 
@@ -278,9 +285,10 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
     r2 = a.r2;
   }
   const int lm = a.lm_type;
-  const int tx = tid % TX, ty = tid / TX;
+  // the thread's cell; a warp without cells keeps the indices of some and owns none
+  const int tx = tid % TX, ty = tid % G::CELLS / TX;
   const int gi = gi0 + tx, gj = gj0 + ty;
-  const bool own = gi <= ix - 2 && gj <= jx - 2;
+  const bool own = tid < G::CELLS && gi <= ix - 2 && gj <= jx - 2;
   const int oc = (ty + 2) * RX + (tx + 2);  // own column in a ring plane
   // dt/dx as dt * (dtx_scale/dx) in the FAST builds (within an ulp), the
   // reference's division in the parity build
@@ -622,7 +630,7 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
       for (int r = lead ? RXY : 0; r <= RXY; ++r) {
         const bool zf = r == RXY;
         const int q = tid + r * NT, n = zf ? 2 : (q < NXF3 ? 0 : 1);
-        if (!zf && q >= NXF3 + NYF3) continue;
+        if (zf ? tid >= G::CELLS : q >= NXF3 + NYF3) continue;
         const int qq = n == 0 ? q : q - NXF3;
         const int fa = n == 0 ? qq % XF : qq % TX, fb = n == 0 ? qq / XF : qq / TX;
         double* const bl = n == 0 ? SLx + fb * XS + fa : SLy + fb * TX + fa;
@@ -811,10 +819,11 @@ int launch_one3d(const StageArgs& a, cudaStream_t s) {
 }
 
 // FP64 HLLD: 16x16 columns, one CTA per SM, or two CTAs of 16x8 columns, the
-// cheaper by the rounds x (planes + prologue) of pick_zchunk; an SM takes 7 %
-// longer for a plane of two 16x8 columns, whose halo is larger (Harris
-// 256x128x256, ms per step: 33.4 with 16x16, 35.9 with 16x8, 34.0 with 32x8), but
-// covers ragged grids better (field loop 100x100x200: 6.5, 5.7, 7.2).
+// cheaper by the rounds x (planes + prologue) of pick_zchunk.  For grids that both
+// cover alike an SM takes longer for a plane of two 16x8 columns, whose halo is
+// larger and with resistivity has corners: 10-12 % on Harris (96x48x96 1.91 against
+// 1.74 ms per step, 256x128x256 32.0 / 28.6), 2 % on the field loop (64x64x128 1.338 /
+// 1.315).  They cover ragged grids better (loop 100x100x200: 5.25 / 5.70).
 template <int FLUX>
 int launch_best3d(const StageArgs& a, cudaStream_t s) {
   int nsm = 0;
@@ -823,7 +832,7 @@ int launch_best3d(const StageArgs& a, cudaStream_t s) {
   double wide = 0.0, small = 0.0;
   pick_zchunk(columns_of<WideCol>(a), a.kx - 2, nsm * WideCol::CTAS, &wide);
   pick_zchunk(columns_of<SmallCol>(a), a.kx - 2, nsm * SmallCol::CTAS, &small);
-  if (1.07 * small < wide) return launch_one3d<double, FLUX, SmallCol>(a, s);
+  if ((a.eta_kind != OMHD_ETA_NONE ? 1.11 : 1.02) * small < wide) return launch_one3d<double, FLUX, SmallCol>(a, s);
   return launch_one3d<double, FLUX, WideCol>(a, s);
 }
 
