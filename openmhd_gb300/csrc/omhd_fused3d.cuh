@@ -61,7 +61,7 @@ using DefaultCol = Col<OMHD_3D_TILE_X, OMHD_3D_TILE_Y, sizeof(T) == 4 ? OMHD_3D_
 // (launch_best3d), with a warp more than the cells need.  The 16x16 plane's 288
 // pairs of face states and 544 x and y faces are 9 and 17 warps' worth, which eight
 // warps did in rounds of 8 and 1: a warp alone on the SM gets a third of the FP64
-// pipe, and a quarter of a plane's time went that way (224 registers and 444 bytes
+// pipe, and a quarter of a plane's time went that way (168 registers with 444 bytes
 // spilled instead of 255; Harris 256x128x256 33.3 -> 28.6 ms per step, two extra
 // warps 28.8, mixed 6.17 -> 6.75: not used there).  16x8: loop 100x100x200 5.70 -> 5.25.
 using WideCol = Col<16, 16, 1, 1>;
