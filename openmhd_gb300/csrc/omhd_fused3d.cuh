@@ -66,6 +66,7 @@ using DefaultCol = Col<OMHD_3D_TILE_X, OMHD_3D_TILE_Y, sizeof(T) == 4 ? OMHD_3D_
 // warps 28.8, mixed 6.17 -> 6.75: not used there).  16x8: loop 100x100x200 5.70 -> 5.25.
 using WideCol = Col<16, 16, 1, 1>;
 using SmallCol = Col<16, 8, 2, 1>;
+using SquareCol = Col<16, 16, 2>;  // FP32-mixed HLLD, beside 32x8 (launch_mixed3d)
 constexpr int NRING = 4;
 constexpr int ZCHUNK = 64;  // most z planes marched by one CTA
 
@@ -836,6 +837,18 @@ int launch_best3d(const StageArgs& a, cudaStream_t s) {
   return launch_one3d<double, FLUX, WideCol>(a, s);
 }
 
+// FP32-mixed HLLD: 16x16 columns where the runs are resistive, whose corner loads the
+// smaller halo saves (Harris, ms per step with 32x8 / 16x16: 64x32x64 0.172 / 0.171,
+// 128x64x128 0.936 / 0.871, 256x128x256 6.18 / 6.07, 512x256x512 51.4 / 51.0), or fewer
+// of them cover the grid (field loop 100x100x200 2.10 / 1.95); else 32x8 (64x64x128 0.442 /
+// 0.460).
+template <int FLUX>
+int launch_mixed3d(const StageArgs& a, cudaStream_t s) {
+  if (a.eta_kind != OMHD_ETA_NONE || columns_of<SquareCol>(a) < columns_of<DefaultCol<float>>(a))
+    return launch_one3d<float, FLUX, SquareCol>(a, s);
+  return launch_one3d<float, FLUX>(a, s);
+}
+
 template <class T>
 int launch_variant3d(const StageArgs& a, cudaStream_t s) {
   switch (a.flux_type) {
@@ -845,6 +858,8 @@ int launch_variant3d(const StageArgs& a, cudaStream_t s) {
     case FX_HLLD:
       if constexpr (OMHD_FAST && sizeof(T) == 8)
         return launch_best3d<FX_HLLD>(a, s);
+      else if constexpr (sizeof(T) == 4)
+        return launch_mixed3d<FX_HLLD>(a, s);
       else
         return launch_one3d<T, FX_HLLD>(a, s);
     default: return launch_one3d<T, FX_LHLLD>(a, s);

@@ -51,3 +51,30 @@ def test_step_vs_oracle(cuda_lib, oracle_mod, nx, ny, nz, wall):
     assert s.sync().status == 0
     g.step(1)
     assert_parity(s.get_state_numpy(), g.U, 1e-12, f"{nx}x{ny}x{nz}")
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(40, 8, 6), (33, 7, 70), (48, 6, 5)])
+@pytest.mark.parametrize("wall", [False, True])
+def test_mixed_columns_agree(cuda_lib, nx, ny, nz, wall):
+    """FP32-mixed: a grid of 32x8 columns, and its state repeated five times along the
+    periodic y axis, which 16x16 columns cover in fewer: the same bits in every copy."""
+    from openmhd_gb300 import Solver, field_loop3d, flip
+
+    columns = lambda n: (-(-nx // 32) * -(-n // 8), -(-nx // 16) * -(-n // 16))  # noqa: E731
+    assert columns(ny)[0] <= columns(ny)[1] and columns(5 * ny)[0] > columns(5 * ny)[1]
+    one, _ = field_loop3d(nx, ny, nz, precision="mixed", limiter="mc")
+    if wall:
+        f = [flip(1, 6), flip(3, 8)]
+        one = dataclasses.replace(one, bc_kind=(1, 1, 0, 0, 1, 1), bc_flip=(f[0], f[0], 0, 0, f[1], f[1]))
+    five = dataclasses.replace(one, jx=5 * ny + 2)
+    U = _state(one, ny)
+    U[:, :, 0], U[:, :, -1] = U[:, :, -2], U[:, :, 1]
+    V = np.concatenate([U[:, :, :1]] + 5 * [U[:, :, 1:-1]] + [U[:, :, -1:]], axis=2)
+    res = []
+    for cfg, state in ((one, U), (five, V)):
+        s = Solver(cfg).put_state(state)
+        s.step(2)
+        assert s.sync().status == 0
+        res.append(s.get_state_numpy())
+    for k in range(5):
+        assert np.array_equal(res[1][:, :, 1 + k * ny : 1 + (k + 1) * ny], res[0][:, :, 1:-1]), k
