@@ -6,7 +6,7 @@ namespace omhd {
 
 // ---------------------------------------------------------------------------
 // FP64 reciprocal and square roots without the FP64 pipe.  That pipe takes one
-// warp instruction in ~16 cycles (an SM issues 64 other ones in that time) and
+// warp instruction in 19 cycles (an SM issues 76 other ones in that time) and
 // bounds the FP64 kernels, so the performance variants (FAST = true) compute
 // 1/x, 1/sqrt(x) and sqrt(x) on the integer pipes: the argument's significand
 // as a 64-bit fixed-point number, a binary32 seed of the special-function unit

@@ -15,16 +15,17 @@ from . import _lib
 from .solver import OmhdError
 
 
-def _ptr(a) -> int:
-    try:
-        import numpy as np
+try:
+    import numpy as _np
+except ImportError:  # pragma: no cover
+    _np = None
 
-        if isinstance(a, np.ndarray):
-            if a.dtype != np.float64 or not a.flags.c_contiguous:
-                raise TypeError("arrays must be C-contiguous float64")
-            return a.ctypes.data
-    except ImportError:  # pragma: no cover
-        pass
+
+def _ptr(a) -> int:
+    if _np is not None and isinstance(a, _np.ndarray):
+        if a.dtype != _np.float64 or not a.flags.c_contiguous:
+            raise TypeError("arrays must be C-contiguous float64")
+        return a.ctypes.data
     import torch
 
     if isinstance(a, torch.Tensor):
@@ -45,7 +46,7 @@ def _dims(U, var_axis: bool = True):
 
 
 def _shape_of(a) -> tuple:
-    return tuple(int(n) for n in a.shape)
+    return tuple(a.shape)
 
 
 def _expect(name: str, a, shape: tuple):
@@ -53,8 +54,8 @@ def _expect(name: str, a, shape: tuple):
     (the library trusts ix/jx/kx and would run past a smaller buffer)."""
     if a is None:
         raise ValueError(f"{name} is required")
-    if _shape_of(a) != tuple(shape):
-        raise ValueError(f"{name} has shape {_shape_of(a)}, expected {tuple(shape)}")
+    if _shape_of(a) != shape:
+        raise ValueError(f"{name} has shape {_shape_of(a)}, expected {shape}")
 
 
 def _planes(nd: int, ix: int, jx: int, kx: int) -> tuple:
@@ -62,28 +63,25 @@ def _planes(nd: int, ix: int, jx: int, kx: int) -> tuple:
 
 
 def _lib_for(*arrays):
+    """The library, its routine calls set to torch's current stream for CUDA tensors and
+    to the default one otherwise."""
     try:
         import torch
-
-        cuda = [a for a in arrays if isinstance(a, torch.Tensor) and a.is_cuda]
-        if cuda:
-            dev = torch.cuda.current_device()
-            bad = [a.device.index for a in cuda if a.device.index != dev]
-            if bad:
-                raise ValueError(f"CUDA tensors must be on the current device cuda:{dev}, got cuda:{bad[0]}")
     except ImportError:  # pragma: no cover
-        pass
+        lib = _lib.load()
+        lib.omhd_set_abort_on_error(0)
+        return lib
+    stream = dev = None
+    for a in arrays:
+        if isinstance(a, torch.Tensor) and a.is_cuda:
+            if dev is None:
+                dev = torch.cuda.current_device()
+                stream = torch.cuda.current_stream(dev).cuda_stream
+            if a.device.index != dev:
+                raise ValueError(f"CUDA tensors must be on the current device cuda:{dev}, got cuda:{a.device.index}")
     lib = _lib.load()
     lib.omhd_set_abort_on_error(0)
-    try:
-        import torch
-
-        if any(isinstance(a, torch.Tensor) and a.is_cuda for a in arrays):
-            lib.omhd_set_stream(C.c_void_p(torch.cuda.current_stream().cuda_stream))
-        else:
-            lib.omhd_set_stream(None)
-    except ImportError:  # pragma: no cover
-        pass
+    lib.omhd_set_stream(stream)
     return lib
 
 
