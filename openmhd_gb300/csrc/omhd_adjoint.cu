@@ -217,7 +217,7 @@ __device__ __forceinline__ void face_vjp(const AdjGeo& g, const double* __restri
 // (columns 1..ix-2, faces 0..jx-2) in the rest; consecutive threads take
 // consecutive cells along x in both.
 template <int MODE>
-__global__ void __launch_bounds__(128) k_adj_faces(AdjGeo g, const double* __restrict__ W,
+__global__ void __launch_bounds__(32) k_adj_faces(AdjGeo g, const double* __restrict__ W,
                                                    const double* __restrict__ lam, const double* __restrict__ lg,
                                                    double lscale, int nbx, const unsigned char* __restrict__ tlim,
                                                    const unsigned short* __restrict__ tface,
@@ -420,7 +420,12 @@ int taped_step(omhd_adjoint* a, int mode, unsigned char* tl, unsigned short* tf)
 int launch_step_vjp(omhd_adjoint* a, const double* Un, const double* U1, const double* lg, double* lam_in,
                     double* lam1, double* lam_out, const unsigned char* tl, const unsigned short* tf) {
   const AdjGeo& g = a->geo;
-  const int TPB = 256, FPB = 128;
+  // Small blocks: an SM holds eight warps of the face kernel (255 registers), which
+  // single ones fill and hand on without waiting for a block's slowest; us per gradient
+  // of 12 steps with face blocks of 128 / 64 / 32 threads: 128x128 4188 / 3990 / 3802,
+  // 300x200 9368 / 9228 / 9223, 512x256 16612 / 16646 / 16617; then cell blocks of 256 /
+  // 64: 3802 / 3735, 9216 / 9128, 16570 / 16450.
+  const int TPB = 64, FPB = 32;
   const int cb = ceil_div((long long)g.n, TPB);
   const int nbx = ceil_div((long long)(g.ix - 1) * (g.jx - 2), FPB);
   const int nby = ceil_div((long long)(g.ix - 2) * (g.jx - 1), FPB);
