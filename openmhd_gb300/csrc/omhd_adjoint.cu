@@ -298,7 +298,10 @@ __global__ void __launch_bounds__(256) k_adj_cells(AdjGeo g, const double* __res
           const double q = recon_weight<0>(g.lm, k);
           gw[v] = fma(1.0 - q, gr, fma(1.0 + q, gl, gw[v]));
         } else {
-          gw[v] = fma(d < 0 ? recon_weight<-1>(g.lm, k) : recon_weight<1>(g.lm, k), gl - gr, gw[v]);
+          const double q = d < 0 ? recon_weight<-1>(g.lm, k) : recon_weight<1>(g.lm, k);
+          // a neighbour that the slope does not depend on gets nothing of an infinite or
+          // NaN gradient either (0 times it would be NaN)
+          gw[v] = fma(q, __double2hiint(q) ? gl - gr : 0.0, gw[v]);
         }
       }
     }
