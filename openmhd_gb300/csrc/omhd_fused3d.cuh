@@ -204,7 +204,7 @@ __device__ __forceinline__ constexpr int rot3(int n, int k) {
 // of the halo tile into ring slot `slot`.
 template <class T, class G>
 __device__ __forceinline__ void load_plane(const StageArgs& a, T* W, int slot, int gk, int gi0, int gj0, bool perx,
-                                           bool pery, bool perz, bool resist, double glmf, bool own_plane) {
+                                           bool pery, bool perz, bool resist, double glmf) {
   constexpr int TX = G::TX, TY = G::TY, NT = G::NT, RX = G::RX, RY = G::RY, PL = G::PL;
   const int ix = a.ix, jx = a.jx, kx = a.kx;
   const size_t N = (size_t)ix * jx * kx;
@@ -231,12 +231,6 @@ __device__ __forceinline__ void load_plane(const StageArgs& a, T* W, int slot, i
     u2v_cell<T, OMHD_FAST, OMHD_FAST && sizeof(T) == 8>(u, f1g, f1g32, ps, w, pr, ro);  // 3D_basic/u2v.f90
 #pragma unroll
     for (int v = 0; v < NV; ++v) Ws[v * PL + q] = w[v];
-    if (own_plane && cx_in && cy_in && gi <= ix - 2 && gj <= jx - 2) {  // u2v.f90:36-45, owner check
-      if (!(pr > 0.0))
-        raise_error(a.err, OMHD_NEG_PRESSURE, gi + 1, gj + 1, gk + 1, 0, pr);
-      else if (!(ro > 0.0))
-        raise_error(a.err, OMHD_NEG_DENSITY, gi + 1, gj + 1, gk + 1, 0, ro);
-    }
   }
 }
 
@@ -324,7 +318,7 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
 
   // ---- prologue: planes k0-2 .. k0+1, then the z face k0-1/2 ----
   for (int p = k0 - 2; p <= k0 + 1; ++p)
-    load_plane<T, G>(a, W, slot(p), p, gi0, gj0, perx, pery, perz, resist, glmf, p == k0);
+    load_plane<T, G>(a, W, slot(p), p, gi0, gj0, perx, pery, perz, resist, glmf);
   __syncthreads();
   T sLc[NV];  // z-upper face state of the current cell (k)
   double Fzp[NV] = {};  // z flux through face k-1/2
@@ -361,7 +355,7 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
       // differently from the loop's; with chunks of ZCHUNK planes it was the first
       // face of a chunk, and keeping it there gives a mixed run the same bits for
       // every split
-      const bool seam = sizeof(T) == 4 && (k - 1) % ZCHUNK == 0;
+      const bool every = (k - 1) % ZCHUNK == 0, seam = sizeof(T) == 4 && every;
       if constexpr (sizeof(T) == 4) {
         if (seam) {
           T L[NV], R[NV], Fo[NV];
@@ -393,18 +387,29 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
         }
       }
       if (k == k0 || seam) __syncthreads();
-      load_plane<T, G>(a, W, slot(k + 2), k + 2, gi0, gj0, perx, pery, perz, resist, glmf, false);
+      load_plane<T, G>(a, W, slot(k + 2), k + 2, gi0, gj0, perx, pery, perz, resist, glmf);
       __syncthreads();
-      if (k > k0) {
-        // positivity of the current plane's own cells (u2v.f90:36-45); plane k0
-        // was checked at load time in the prologue
-        if (own) {
-          const double ro = to_f64<T>(Wv(k, RO, oc)), pr = to_f64<T>(Wv(k, PR, oc));
-          if (pr <= 0)
-            raise_error(a.err, OMHD_NEG_PRESSURE, gi + 1, gj + 1, k + 1, 0, pr);
-          else if (ro <= 0)
-            raise_error(a.err, OMHD_NEG_DENSITY, gi + 1, gj + 1, k + 1, 0, ro);
+      // positivity of the plane's own cells (u2v.f90:36-45).  NaN counts on every
+      // ZCHUNK-th plane, where the FP32 build also judges the FP64 values: wherever the
+      // chunks begin, so that which states a run refuses does not depend on the cut
+      if (own) {
+        double ro, pr;
+        if (seam) {
+          double u[NV];
+          T w[NV];
+          const size_t c = (size_t)gi + (size_t)ix * ((size_t)gj + (size_t)jx * k);
+#pragma unroll
+          for (int v = 0; v < NV; ++v) u[v] = a.Uin[v * N + c];
+          u2v_cell<T, OMHD_FAST, OMHD_FAST && sizeof(T) == 8>(u, a.gm1, a.gm1_f, u[PS], w, pr, ro);
+        } else {
+          ro = to_f64<T>(Wv(k, RO, oc));
+          pr = to_f64<T>(Wv(k, PR, oc));
         }
+        auto refused = [&](double x) { return !gt0_<true>(x) && (every || x == x); };
+        if (refused(pr))
+          raise_error(a.err, OMHD_NEG_PRESSURE, gi + 1, gj + 1, k + 1, 0, pr);
+        else if (refused(ro))
+          raise_error(a.err, OMHD_NEG_DENSITY, gi + 1, gj + 1, k + 1, 0, ro);
       }
       const T* Wk = W + (size_t)slot(k) * NV * PL;
 
