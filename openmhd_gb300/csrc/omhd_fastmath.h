@@ -213,7 +213,21 @@ __device__ __forceinline__ double mul_int(double a, double b, bool& bad) {
   return __hiloint2double((int)rh, (int)rl);
 }
 
-// x / 2 by its exponent (exact; results below 2^-1022 become signed zeros)
+// x / 2, rounded to nearest: the IEEE result for all arguments, by the exponent or,
+// below 2^-1021, where the bits of |x| are its value in units of 2^-1074 (exponent field
+// included), as an integer, to even.  Written out with one select a word: as half_exact
+// with a second select the mixed 3D kernel took 0.5 to 1.3 % longer (Harris 256x128x256,
+// 14.02-14.13 ms for 2 steps, against 13.94; without the integer halves 13.93).
+__device__ __forceinline__ double half_rn(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), mh = hi & 0x7fffffffu, lo = (unsigned)__double2loint(x);
+  const unsigned long long m =
+      (((unsigned long long)(mh >> 1) << 32) | __funnelshift_r(lo, mh, 1)) + (lo & (lo >> 1) & 1u);
+  const bool tiny = mh < 0x00200000u;
+  const unsigned h = mh >= 0x7ff00000u ? hi : hi - 0x00100000u;  // infinity and NaN stay
+  return __hiloint2double((int)(tiny ? (unsigned)(m >> 32) | (hi & 0x80000000u) : h), (int)(tiny ? (unsigned)m : lo));
+}
+
+// its exponent part alone (probed; exact; results below 2^-1022 become signed zeros)
 __device__ __forceinline__ double half_exact(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), e = hi & 0x7ff00000u;
   const bool tiny = e < 0x00200000u;

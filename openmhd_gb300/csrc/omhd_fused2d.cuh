@@ -702,7 +702,7 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
     // instruction holds the FP64 pipe like any other, and with the choices inside
     // the ensemble kernel spent half of its FP64 time on the results not taken.
     // Mixed: the differences of binary32 fluxes and the halving are made on the FP32
-    // and integer pipes (sub_f32, half_exact: the same bits), 18 of the 54 FP64
+    // and integer pipes (sub_f32, half_rn: the same bits), 18 of the 54 FP64
     // operations of a cell in stage 1 and 27 of 74 in stage 2; KH 2048x1024: 338 to
     // 299 and 452 to 378 us, the FP64 pipe 55 to 42 % busy, issue slots 50 to 60 %.
     auto dF = [&](int v) {  // F(i-1/2) - F(i+1/2) in FP64
@@ -728,7 +728,7 @@ __device__ __forceinline__ double phase_update(const StageArgs& a, int bxi, int 
       } else {
 #pragma unroll
         for (int v = 0; v < NV; ++v)
-          out[v] = half_exact(fma(dtx, fma(ryx, dG(v), dF(v)), ub(v) + U1[v * N + c]));
+          out[v] = half_rn(fma(dtx, fma(ryx, dG(v), dF(v)), ub(v) + U1[v * N + c]));
       }
     } else {
       double d[NV];

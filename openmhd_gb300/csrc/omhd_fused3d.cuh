@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
           for (int v = 0; v < NV; ++v) out[v] = fma(dtx, d(v), ub(v));
         } else {
 #pragma unroll
-          for (int v = 0; v < NV; ++v) out[v] = half_exact(fma(dtx, d(v), ub(v) + a.U1[v * N + c]));
+          for (int v = 0; v < NV; ++v) out[v] = half_rn(fma(dtx, d(v), ub(v) + a.U1[v * N + c]));
         }
       } else {
         double d[NV];

@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(NTOT, 1) k_stage3d_pipe(const StageArgs a) {
           const bool rk2 = a.stage == 1 || a.time_type == OMHD_TIME_RK2;
           const double u0 = rk2 ? ub : ub + a.U1[v * N + cc0];
           const double d = fma(dtx, fma(a.rzx, fzm - fzp, fma(a.ryx, gm - gp, acc)), u0);
-          out[v] = rk2 ? d : half_exact(d);
+          out[v] = rk2 ? d : half_rn(d);
         }
         if (a.stage == 2) out[PS] = glmf * out[PS];
         int xt[3], yt[3], zt[3], xf[3], yf[3], zf[3], nxt = 1, nyt = 1, nzt = 1;

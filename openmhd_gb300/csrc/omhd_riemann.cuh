@@ -133,7 +133,7 @@ __device__ __forceinline__ double sub_f64(T a, T b) {
 // x / 2, by the exponent in the FAST builds
 template <bool FAST>
 __device__ __forceinline__ double half_(double x) {
-  return FAST ? half_exact(x) : 0.5 * x;
+  return FAST ? half_rn(x) : 0.5 * x;
 }
 
 enum { LM_FLAT = 0, LM_MINMOD = 1, LM_MC = 2, LM_VANLEER = 3, LM_KOREN = 4 };
