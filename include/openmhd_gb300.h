@@ -284,6 +284,11 @@ typedef struct {
   uint64_t seed;       /* seeded deviates (SplitMix64) */
 } omhd_model;
 
+/* How the stage kernels cut this configuration's grid on a device with `sms` SMs
+ * (no counterpart in the reference): the cells of a tile or column in x and y, the
+ * z planes that a thread block marches (1 in 2D) and the blocks per SM that the
+ * build is made for.  Host code only: needs no GPU. */
+int omhd_probe_tiling(const omhd_config* cfg, int sms, int tile[4]);
 int omhd_solver_create(const omhd_config* cfg, omhd_solver** out);
 int omhd_solver_destroy(omhd_solver* s);
 /* stream for all work of this handle (NULL = the legacy default stream) */

@@ -101,6 +101,7 @@ SIGNATURES = [
     ("omhd_probe_fastmath", I, [P, C.c_longlong, P]),
     ("omhd_probe_mul", I, [P, P, C.c_longlong, P]),
     ("omhd_probe_convert", I, [P, P, P, P, C.c_longlong]),
+    ("omhd_probe_tiling", I, [C.POINTER(Config), I, c_int_p]),
     ("omhd_solver_create", I, [C.POINTER(Config), C.POINTER(C.c_void_p)]),
     ("omhd_solver_destroy", I, [P]),
     ("omhd_solver_set_stream", I, [P, P]),

@@ -113,6 +113,20 @@ int launch_stage3d_fp64(const StageArgs& a, cudaStream_t s);
 int launch_stage3d_parity(const StageArgs& a, cudaStream_t s);
 int launch_stage3d_mixed(const StageArgs& a, cudaStream_t s);
 
+// How a stage kernel cuts the grid described by a (ix, jx, kx, nd, lm_type, flux_type,
+// eta_kind) on a device with nsm SMs: the cells of a tile or column in x and y, the z
+// planes a CTA marches (1 in 2D) and the CTAs per SM of the build that runs.  The
+// launchers take their decisions from the functions behind these.
+struct Tiling {
+  int tx, ty, tz, ctas;
+};
+Tiling tiling2d_fp64(const StageArgs& a, int nsm);
+Tiling tiling2d_parity(const StageArgs& a, int nsm);
+Tiling tiling2d_mixed(const StageArgs& a, int nsm);
+Tiling tiling3d_fp64(const StageArgs& a, int nsm);
+Tiling tiling3d_parity(const StageArgs& a, int nsm);
+Tiling tiling3d_mixed(const StageArgs& a, int nsm);
+
 // SMs of the current device
 inline int sm_count(int* nsm) {
   int dev = 0;

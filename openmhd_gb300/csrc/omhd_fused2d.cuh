@@ -1045,6 +1045,10 @@ inline int pick_rows(int ntx, int ny, int nsm) {
   return best;
 }
 
+inline Tiling tiling_pipe(const StageArgs& a, int nsm) {
+  return {PipeGeo::TX, pick_rows((a.ix - 2 + PipeGeo::TX - 1) / PipeGeo::TX, a.jx - 2, nsm), 1, 1};
+}
+
 template <int FLUX, int TAPE, int NPW = OMHD_PIPE_PRODUCER_WARPS>
 int launch_pipe(const StageArgs& a, cudaStream_t s) {
   const size_t bytes = pipe_smem_bytes_tma();
@@ -1055,7 +1059,7 @@ int launch_pipe(const StageArgs& a, cudaStream_t s) {
   r = sm_count(&nsm);
   if (r) return r;
   const int ntx = (a.ix - 2 + PipeGeo::TX - 1) / PipeGeo::TX;
-  const int ty = pick_rows(ntx, a.jx - 2, nsm);
+  const int ty = tiling_pipe(a, nsm).ty;
   const int ntiles = ntx * ((a.jx - 2 + ty - 1) / ty);
   const int grid = ntiles < nsm ? ntiles : nsm;
   // the tensor map of this stage's input state (encoded on the host, passed by
@@ -1161,6 +1165,11 @@ int launch_ctas(const StageArgs& a, dim3 grid, cudaStream_t s) {
 // than one round of four.  ms a step with four / five: 64^2 0.0295 / 0.0299, 256^2
 // (512 tiles on 152 SMs) 0.0481 / 0.0490, 700^2 0.2080 / 0.2063, 1000x500 0.2129 /
 // 0.2027, 2048x1024 0.784 / 0.749, 4096x2048 2.960 / 2.855.
+inline bool five_ctas(const StageArgs& a, int nsm) {
+  using G = GeoFor<float>::type;
+  const long long tiles = (long long)((a.ix - 2 + G::TX - 1) / G::TX) * ((a.jx - 2 + G::TY - 1) / G::TY);
+  return a.flux_type == FX_HLLD && tiles > (long long)OMHD_MIXED_MIN_CTAS * nsm;
+}
 template <class T, int FLUX, int TAPE = tape::kNone>
 int launch_one(const StageArgs& a, cudaStream_t s) {
   using G = typename GeoFor<T>::type;
@@ -1170,13 +1179,17 @@ int launch_one(const StageArgs& a, cudaStream_t s) {
       int nsm = 0;
       const int r = sm_count(&nsm);
       if (r) return r;
-      if ((long long)grid.x * grid.y > (long long)OMHD_MIXED_MIN_CTAS * nsm)
-        return launch_ctas<T, FLUX, TAPE, OMHD_MIXED_MIN_CTAS + 1>(a, grid, s);
+      if (five_ctas(a, nsm)) return launch_ctas<T, FLUX, TAPE, OMHD_MIXED_MIN_CTAS + 1>(a, grid, s);
     }
     return launch_ctas<T, FLUX, TAPE, OMHD_MIXED_MIN_CTAS>(a, grid, s);
   } else {
     return launch_ctas<T, FLUX, TAPE, 1>(a, grid, s);
   }
+}
+template <class T>
+Tiling tiling_one(const StageArgs& a, int nsm) {
+  using G = typename GeoFor<T>::type;
+  return {G::TX, G::TY, 1, sizeof(T) == 4 ? OMHD_MIXED_MIN_CTAS + (five_ctas(a, nsm) ? 1 : 0) : 1};
 }
 
 template <class T, int FLUX, class G>

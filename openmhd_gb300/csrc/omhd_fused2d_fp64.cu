@@ -11,8 +11,16 @@ int fill_eta2d_fp64(const StageArgs& a, double* etax, double* etay, cudaStream_t
 // HLLD with minmod or MC runs the tape-recording instantiation with recording
 // switched off (null tape pointers): one machine code for the plain and the
 // recording step, so a recorded run reproduces a plain run bit for bit.
+namespace {
+bool taped_scheme(const StageArgs& a) {
+  return a.flux_type == FX_HLLD && (a.lm_type == LM_MINMOD || a.lm_type == LM_MC);
+}
+}  // namespace
+Tiling tiling2d_fp64(const StageArgs& a, int nsm) {
+  return taped_scheme(a) && pipe2d_enabled() ? v_fp64::tiling_pipe(a, nsm) : v_fp64::tiling_one<double>(a, nsm);
+}
 int launch_stage2d_fp64(const StageArgs& a, cudaStream_t s) {
-  if (a.flux_type == FX_HLLD && (a.lm_type == LM_MINMOD || a.lm_type == LM_MC)) {
+  if (taped_scheme(a)) {
     StageArgs b = a;
     b.tlim = nullptr;
     b.tface = nullptr;

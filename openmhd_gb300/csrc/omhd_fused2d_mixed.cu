@@ -8,6 +8,7 @@ namespace omhd {
 int fill_eta2d_mixed(const StageArgs& a, double* etax, double* etay, cudaStream_t s) {
   return v_mixed::fill_eta2d(a, etax, etay, s);
 }
+Tiling tiling2d_mixed(const StageArgs& a, int nsm) { return v_mixed::tiling_one<float>(a, nsm); }
 int launch_stage2d_mixed(const StageArgs& a, cudaStream_t s) { return v_mixed::launch_variant<float>(a, s); }
 }  // namespace omhd
 

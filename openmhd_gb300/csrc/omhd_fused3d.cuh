@@ -58,7 +58,7 @@ struct Col {
 template <class T>
 using DefaultCol = Col<OMHD_3D_TILE_X, OMHD_3D_TILE_Y, sizeof(T) == 4 ? OMHD_3D_MIXED_MIN_CTAS : 1>;
 // FP64 HLLD with fused multiply-adds: 16x16, or two 16x8 CTAs per SM
-// (launch_best3d), with a warp more than the cells need.  The 16x16 plane's 288
+// (small_columns), with a warp more than the cells need.  The 16x16 plane's 288
 // pairs of face states and 544 x and y faces are 9 and 17 warps' worth, which eight
 // warps did in rounds of 8 and 1: a warp alone on the SM gets a third of the FP64
 // pipe, and a quarter of a plane's time went that way (168 registers with 444 bytes
@@ -66,7 +66,7 @@ using DefaultCol = Col<OMHD_3D_TILE_X, OMHD_3D_TILE_Y, sizeof(T) == 4 ? OMHD_3D_
 // warps 28.8, mixed 6.17 -> 6.75: not used there).  16x8: loop 100x100x200 5.70 -> 5.25.
 using WideCol = Col<16, 16, 1, 1>;
 using SmallCol = Col<16, 8, 2, 1>;
-using SquareCol = Col<16, 16, 2>;  // FP32-mixed HLLD, beside 32x8 (launch_mixed3d)
+using SquareCol = Col<16, 16, 2>;  // FP32-mixed HLLD, beside 32x8 (square_columns)
 constexpr int NRING = 4;
 constexpr int ZCHUNK = 64;  // most z planes marched by one CTA
 
@@ -810,6 +810,11 @@ inline long long columns_of(const StageArgs& a) {
   return (long long)((a.ix - 2 + G::TX - 1) / G::TX) * ((a.jx - 2 + G::TY - 1) / G::TY);
 }
 
+template <class G>
+Tiling tiling_of(const StageArgs& a, int nsm) {
+  return {G::TX, G::TY, pick_zchunk(columns_of<G>(a), a.kx - 2, nsm * G::CTAS), G::CTAS};
+}
+
 template <class T, int FLUX, class G = DefaultCol<T>>
 int launch_one3d(const StageArgs& a, cudaStream_t s) {
   const size_t bytes = G::template smem_bytes<T>();
@@ -818,7 +823,7 @@ int launch_one3d(const StageArgs& a, cudaStream_t s) {
   int nsm = 0;
   if (!r) r = sm_count(&nsm);
   if (r) return r;
-  const int zc = pick_zchunk(columns_of<G>(a), a.kx - 2, nsm * G::CTAS);
+  const int zc = tiling_of<G>(a, nsm).tz;
   dim3 grid((a.ix - 2 + G::TX - 1) / G::TX, (a.jx - 2 + G::TY - 1) / G::TY, (a.kx - 2 + zc - 1) / zc);
   k_stage3d<T, FLUX, G><<<grid, G::NT, bytes, s>>>(a, zc);
   return (int)cudaGetLastError();
@@ -830,16 +835,11 @@ int launch_one3d(const StageArgs& a, cudaStream_t s) {
 // larger and with resistivity has corners: 10-12 % on Harris (96x48x96 1.91 against
 // 1.74 ms per step, 256x128x256 32.0 / 28.6), 2 % on the field loop (64x64x128 1.338 /
 // 1.315).  They cover ragged grids better (loop 100x100x200: 5.25 / 5.70).
-template <int FLUX>
-int launch_best3d(const StageArgs& a, cudaStream_t s) {
-  int nsm = 0;
-  const int r = sm_count(&nsm);
-  if (r) return r;
+inline bool small_columns(const StageArgs& a, int nsm) {
   double wide = 0.0, small = 0.0;
   pick_zchunk(columns_of<WideCol>(a), a.kx - 2, nsm * WideCol::CTAS, &wide);
   pick_zchunk(columns_of<SmallCol>(a), a.kx - 2, nsm * SmallCol::CTAS, &small);
-  if ((a.eta_kind != OMHD_ETA_NONE ? 1.11 : 1.02) * small < wide) return launch_one3d<double, FLUX, SmallCol>(a, s);
-  return launch_one3d<double, FLUX, WideCol>(a, s);
+  return (a.eta_kind != OMHD_ETA_NONE ? 1.11 : 1.02) * small < wide;
 }
 
 // FP32-mixed HLLD: 16x16 columns where the runs are resistive, whose corner loads the
@@ -847,11 +847,26 @@ int launch_best3d(const StageArgs& a, cudaStream_t s) {
 // 128x64x128 0.936 / 0.871, 256x128x256 6.18 / 6.07, 512x256x512 51.4 / 51.0), or fewer
 // of them cover the grid (field loop 100x100x200 2.10 / 1.95); else 32x8 (64x64x128 0.442 /
 // 0.460).
-template <int FLUX>
-int launch_mixed3d(const StageArgs& a, cudaStream_t s) {
-  if (a.eta_kind != OMHD_ETA_NONE || columns_of<SquareCol>(a) < columns_of<DefaultCol<float>>(a))
-    return launch_one3d<float, FLUX, SquareCol>(a, s);
-  return launch_one3d<float, FLUX>(a, s);
+inline bool square_columns(const StageArgs& a) {
+  return a.eta_kind != OMHD_ETA_NONE || columns_of<SquareCol>(a) < columns_of<DefaultCol<float>>(a);
+}
+
+// calls f with the column of an HLLD launch of face arithmetic T
+template <class T, class F>
+auto with_hlld_column(const StageArgs& a, int nsm, F&& f) {
+  if constexpr (OMHD_FAST && sizeof(T) == 8) {
+    return small_columns(a, nsm) ? f(SmallCol{}) : f(WideCol{});
+  } else if constexpr (sizeof(T) == 4) {
+    return square_columns(a) ? f(SquareCol{}) : f(DefaultCol<float>{});
+  } else {
+    return f(DefaultCol<T>{});
+  }
+}
+
+template <class T>
+Tiling tiling3d(const StageArgs& a, int nsm) {
+  if (a.flux_type != FX_HLLD) return tiling_of<DefaultCol<T>>(a, nsm);
+  return with_hlld_column<T>(a, nsm, [&](auto col) { return tiling_of<decltype(col)>(a, nsm); });
 }
 
 template <class T>
@@ -860,13 +875,12 @@ int launch_variant3d(const StageArgs& a, cudaStream_t s) {
     case FX_LLF: return launch_one3d<T, FX_LLF>(a, s);
     case FX_HLL: return launch_one3d<T, FX_HLL>(a, s);
     case FX_HLLC: return launch_one3d<T, FX_HLLC>(a, s);
-    case FX_HLLD:
-      if constexpr (OMHD_FAST && sizeof(T) == 8)
-        return launch_best3d<FX_HLLD>(a, s);
-      else if constexpr (sizeof(T) == 4)
-        return launch_mixed3d<FX_HLLD>(a, s);
-      else
-        return launch_one3d<T, FX_HLLD>(a, s);
+    case FX_HLLD: {
+      int nsm = 0;
+      const int r = sm_count(&nsm);
+      if (r) return r;
+      return with_hlld_column<T>(a, nsm, [&](auto col) { return launch_one3d<T, FX_HLLD, decltype(col)>(a, s); });
+    }
     default: return launch_one3d<T, FX_LHLLD>(a, s);
   }
 }

@@ -5,5 +5,6 @@
 #include "omhd_fused3d.cuh"
 
 namespace omhd {
+Tiling tiling3d_mixed(const StageArgs& a, int nsm) { return v_mixed::d3::tiling3d<float>(a, nsm); }
 int launch_stage3d_mixed(const StageArgs& a, cudaStream_t s) { return v_mixed::d3::launch_variant3d<float>(a, s); }
 }  // namespace omhd

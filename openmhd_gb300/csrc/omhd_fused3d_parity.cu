@@ -5,5 +5,6 @@
 #include "omhd_fused3d.cuh"
 
 namespace omhd {
+Tiling tiling3d_parity(const StageArgs& a, int nsm) { return v_parity::d3::tiling3d<double>(a, nsm); }
 int launch_stage3d_parity(const StageArgs& a, cudaStream_t s) { return v_parity::d3::launch_variant3d<double>(a, s); }
 }  // namespace omhd

@@ -473,6 +473,29 @@ int omhd_solver_create(const omhd_config* cfg, omhd_solver** out) {
   return OMHD_OK;
 }
 
+int omhd_probe_tiling(const omhd_config* cfg, int sms, int tile[4]) {
+  const int r = validate(cfg);
+  if (r) return r;
+  if (sms <= 0 || !tile) return OMHD_BAD_ARG;
+  StageArgs a;
+  memset(&a, 0, sizeof a);
+  a.ix = cfg->ix;
+  a.jx = cfg->jx;
+  a.kx = cfg->kx;
+  a.nd = cfg->nd;
+  a.lm_type = cfg->lm_type;
+  a.flux_type = cfg->flux_type;
+  a.eta_kind = cfg->eta_kind;
+  Tiling (*const of[2][3])(const StageArgs&, int) = {{tiling2d_fp64, tiling2d_parity, tiling2d_mixed},
+                                                     {tiling3d_fp64, tiling3d_parity, tiling3d_mixed}};
+  const Tiling t = of[cfg->nd - 2][cfg->precision](a, sms);
+  tile[0] = t.tx;
+  tile[1] = t.ty;
+  tile[2] = t.tz;
+  tile[3] = t.ctas;
+  return OMHD_OK;
+}
+
 int omhd_solver_destroy(omhd_solver* s) {
   if (!s) return OMHD_OK;
   drop_graph(s);
