@@ -842,13 +842,22 @@ inline bool small_columns(const StageArgs& a, int nsm) {
   return (a.eta_kind != OMHD_ETA_NONE ? 1.11 : 1.02) * small < wide;
 }
 
-// FP32-mixed HLLD: 16x16 columns where the runs are resistive, whose corner loads the
-// smaller halo saves (Harris, ms per step with 32x8 / 16x16: 64x32x64 0.172 / 0.171,
-// 128x64x128 0.936 / 0.871, 256x128x256 6.18 / 6.07, 512x256x512 51.4 / 51.0), or fewer
-// of them cover the grid (field loop 100x100x200 2.10 / 1.95); else 32x8 (64x64x128 0.442 /
-// 0.460).
-inline bool square_columns(const StageArgs& a) {
-  return a.eta_kind != OMHD_ETA_NONE || columns_of<SquareCol>(a) < columns_of<DefaultCol<float>>(a);
+// FP32-mixed HLLD.  Resistive runs: 16x16 columns, whose smaller halo saves corner loads,
+// unless 32x8 columns cover the grid in fewer rounds x (planes + prologue), as they do
+// where ny is no multiple of 16: half of a 16x16 column's faces may then be outside the
+// grid and are solved all the same.  Harris-type grids, us per step with 32x8 / 16x16:
+// 1024x8x1024 6585 / 11306, 512x24x512 5018 / 6399, 512x40x512 8373 / 9540, 300x72x300
+// 5476 / 5725; at equal cost 128x64x128 934 / 870, 256x128x256 6605 / 6475, 512x256x512
+// 51304 / 50946, 96x48x96 393 / 394 (48x24x200 272 / 300, the worst of 25 grids).  Other
+// runs: 16x16 only where fewer of them cover the grid (field loop 100x100x200 2130 /
+// 1949, 64x64x128 449 / 473).
+inline bool square_columns(const StageArgs& a, int nsm) {
+  using Flat = DefaultCol<float>;
+  if (a.eta_kind == OMHD_ETA_NONE) return columns_of<SquareCol>(a) < columns_of<Flat>(a);
+  double square = 0.0, flat = 0.0;
+  pick_zchunk(columns_of<SquareCol>(a), a.kx - 2, nsm * SquareCol::CTAS, &square);
+  pick_zchunk(columns_of<Flat>(a), a.kx - 2, nsm * Flat::CTAS, &flat);
+  return square <= flat;
 }
 
 // calls f with the column of an HLLD launch of face arithmetic T
@@ -857,7 +866,7 @@ auto with_hlld_column(const StageArgs& a, int nsm, F&& f) {
   if constexpr (OMHD_FAST && sizeof(T) == 8) {
     return small_columns(a, nsm) ? f(SmallCol{}) : f(WideCol{});
   } else if constexpr (sizeof(T) == 4) {
-    return square_columns(a) ? f(SquareCol{}) : f(DefaultCol<float>{});
+    return square_columns(a, nsm) ? f(SquareCol{}) : f(DefaultCol<float>{});
   } else {
     return f(DefaultCol<T>{});
   }

@@ -91,6 +91,26 @@ def test_columns_3d_fp64(tiling, sms, resistive):
         assert tiling(_cfg(n, "fp64_parity", resistive), sms) == default
 
 
+@pytest.mark.parametrize("sms", SMS)
+@pytest.mark.parametrize("resistive", [False, True])
+def test_columns_3d_mixed(tiling, sms, resistive):
+    """Also thin grids, of which 16x16 columns would leave half outside: never the column
+    with the higher cost."""
+    thin = [(1024, 8, 1024), (512, 8, 512), (512, 24, 512), (512, 40, 512), (128, 8, 128), (300, 72, 300), (700, 8, 50)]
+    for n in GRIDS_3D + thin:
+        (square, a), (flat, b) = _columns(n, 16, 16, 2, sms), _columns(n, 32, 8, 2, sms)
+        if resistive:
+            want = a if square <= flat else b
+        else:
+            want = a if _up(n[0], 16) * _up(n[1], 16) < _up(n[0], 32) * _up(n[1], 8) else b
+        got = tiling(_cfg(n, "mixed", resistive), sms)
+        assert got == want, n
+        assert (square if got[0] == 16 else flat) == min(square, flat), n
+        assert tiling(_cfg(n, "mixed", resistive, flux="llf"), sms) == b
+    if sms == 152 and resistive:
+        assert all(tiling(_cfg(n, "mixed", True), sms)[:2] == (32, 8) for n in thin)
+
+
 def test_column_grids_take_both(tiling):
     assert {tiling(_cfg(n, "fp64", r), 152)[1] for n, r in itertools.product(COLUMN_GRIDS, (False, True))} == {8, 16}
 
