@@ -525,13 +525,7 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
                 auto B = [&](int var, int dxo, int dyo, int dzo) { return to_f64<T>(Wv(k + dzo, var, o + dxo + dyo * RX)); };
                 const double eta_dx = sep_eta ? harris_eta_dx<double>(ex_f[fx], ez_c[k - k0 + 1], inv_dx)
                                               : eta3(a.eta_kind, a.xc[g] + 0.5 * a.dx, a.yc[gjj], a.zc[k]) / a.dx;
-                const double JyS = -(B(BZ, 1, 0, 0) - B(BZ, 0, 0, 0)) +
-                                   0.25 * (B(BX, 0, 0, 1) + B(BX, 1, 0, 1) - B(BX, 0, 0, -1) - B(BX, 1, 0, -1));
-                const double JzS = (B(BY, 1, 0, 0) - B(BY, 0, 0, 0)) -
-                                   0.25 * (B(BX, 0, 1, 0) + B(BX, 1, 1, 0) - B(BX, 0, -1, 0) - B(BX, 1, -1, 0));
-                Fo[EN] = Fo[EN] + 0.5 * eta_dx * (JyS * (B(BZ, 0, 0, 0) + B(BZ, 1, 0, 0)) - JzS * (B(BY, 0, 0, 0) + B(BY, 1, 0, 0)));
-                Fo[BY] = Fo[BY] - eta_dx * JzS;
-                Fo[BZ] = Fo[BZ] + eta_dx * JyS;
+                resist_face_f64<0>(B, eta_dx, Fo);
               }
             }
           }
@@ -560,13 +554,7 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
                 auto B = [&](int var, int dxo, int dyo, int dzo) { return to_f64<T>(Wv(k + dzo, var, o + dxo + dyo * RX)); };
                 const double eta_dx = sep_eta ? harris_eta_dx<double>(ex_c[cx + 1], ez_c[k - k0 + 1], inv_dx)
                                               : eta3(a.eta_kind, a.xc[gii], a.yc[g] + 0.5 * a.dx, a.zc[k]) / a.dx;
-                const double JxS = (B(BZ, 0, 1, 0) - B(BZ, 0, 0, 0)) -
-                                   0.25 * (B(BY, 0, 0, 1) + B(BY, 0, 1, 1) - B(BY, 0, 0, -1) - B(BY, 0, 1, -1));
-                const double JzS = -(B(BX, 0, 1, 0) - B(BX, 0, 0, 0)) +
-                                   0.25 * (B(BY, 1, 0, 0) + B(BY, 1, 1, 0) - B(BY, -1, 0, 0) - B(BY, -1, 1, 0));
-                Fo[EN] = Fo[EN] + 0.5 * eta_dx * (JzS * (B(BX, 0, 0, 0) + B(BX, 0, 1, 0)) - JxS * (B(BZ, 0, 0, 0) + B(BZ, 0, 1, 0)));
-                Fo[BX] = Fo[BX] + eta_dx * JzS;
-                Fo[BZ] = Fo[BZ] - eta_dx * JxS;
+                resist_face_f64<1>(B, eta_dx, Fo);
               }
             }
           }
@@ -616,13 +604,7 @@ __global__ void __launch_bounds__(G::NT, G::CTAS) k_stage3d(const StageArgs a, c
           auto B = [&](int var, int dxo, int dyo, int dzo) { return to_f64<T>(Wv(k + dzo, var, oc + dxo + dyo * RX)); };
           const double eta_dx = sep_eta ? harris_eta_dx<double>(ex_c[tx + 1], ez_f[k - k0 + 1], inv_dx)
                                         : eta3(a.eta_kind, a.xc[gi], a.yc[gj], a.zc[k] + 0.5 * a.dx) / a.dx;
-          const double JyS = (B(BX, 0, 0, 1) - B(BX, 0, 0, 0)) -
-                             0.25 * (B(BZ, 1, 0, 0) + B(BZ, 1, 0, 1) - B(BZ, -1, 0, 0) - B(BZ, -1, 0, 1));
-          const double JxS = -(B(BY, 0, 0, 1) - B(BY, 0, 0, 0)) +
-                             0.25 * (B(BZ, 0, 1, 0) + B(BZ, 0, 1, 1) - B(BZ, 0, -1, 0) - B(BZ, 0, -1, 1));
-          Fzc[EN] = Fzc[EN] + 0.5 * eta_dx * (JxS * (B(BY, 0, 0, 0) + B(BY, 0, 0, 1)) - JyS * (B(BX, 0, 0, 0) + B(BX, 0, 0, 1)));
-          Fzc[BX] = Fzc[BX] - eta_dx * JyS;
-          Fzc[BY] = Fzc[BY] + eta_dx * JxS;
+          resist_face_f64<2>(B, eta_dx, Fzc);
         }
       }
     };
