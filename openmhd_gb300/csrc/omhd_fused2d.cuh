@@ -572,9 +572,9 @@ __device__ __forceinline__ void phase_flux_rot(const StageArgs& a, int bxi, int 
 // warps) and all y faces (items NXFP..NXFP+NYF-1)
 template <class T, int FLUX, class G, int TAPE>
 __device__ __forceinline__ void phase_flux(const StageArgs& a, int bxi, int byi, const TileMem<T>& m, int t, int n,
-                                           const StageScalars<T>& ks, const int ty = G::TY) {
+                                           const StageScalars<T>& ks) {
   if constexpr (OMHD_FAST && sizeof(T) == 8) {
-    phase_flux_rot<T, FLUX, G, TAPE>(a, bxi, byi, m, t, n, ks, ty);
+    phase_flux_rot<T, FLUX, G, TAPE>(a, bxi, byi, m, t, n, ks, G::TY);
     return;
   }
   constexpr int TX = G::TX, RX = G::RX;
@@ -1001,7 +1001,7 @@ __global__ void __launch_bounds__(NPW * 32 + PipeGeo::NT, 1)
       const TileMem<double> m = pipe_mem(smem_raw, b, resist);
       if (i >= 1) named_bar_sync(kPipeBarFull + b, NTOT);
       const float known = a.stage == 2 ? cfl_known(st) : 0.0f;
-      phase_flux<double, FLUX, G, TAPE>(a, w % ntx, w / ntx, m, t, NC, ks, ty);
+      phase_flux_rot<double, FLUX, G, TAPE>(a, w % ntx, w / ntx, m, t, NC, ks, ty);
       named_bar_sync(kPipeBarCons, NC);
       const double v = phase_update<double, G>(a, w % ntx, w / ntx, m, t, NC, ks, known, ty);
       if (a.stage == 2) cfl_publish(st, v, known);
