@@ -212,8 +212,8 @@ void omhd_set_tma_staging(int enable);
  * selects the warp-specialised kernel (same scheme; results agree to
  * rounding).  Library-global: set it before stepping, from one thread. */
 void omhd_set_3d_pipeline(int enable);
-/* The warp-specialised FP64 2D stage kernel (HLLD with minmod or MC, no
- * resistivity; no counterpart in the reference): on by default; 0 selects the
+/* The warp-specialised FP64 2D stage kernel (HLLD with minmod or MC; no
+ * counterpart in the reference): on by default; 0 selects the
  * one-role 2D kernel (same scheme; results agree to rounding), for
  * comparisons.  Library-global: set it before stepping, from one thread. */
 void omhd_set_2d_pipeline(int enable);

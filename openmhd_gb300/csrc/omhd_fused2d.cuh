@@ -238,8 +238,8 @@ __device__ __forceinline__ void phase_load(const StageArgs& a, int bxi, int byi,
   const float f1g32 = a.gm1_f;
   T* W = m.W;
   // FP64: two cells per pass, both cells' loads issued before either is
-  // converted, so their global-memory latencies overlap; FP32-mixed (two CTAs
-  // per SM, 112 registers) one cell per pass
+  // converted, so their global-memory latencies overlap; FP32-mixed (72 or 96
+  // registers, other CTAs to overlap with) one cell per pass
   constexpr int B = sizeof(T) == 8 ? 2 : 1;
 #pragma unroll 1
   for (int q0 = t; q0 < nq; q0 += B * n) {

@@ -763,7 +763,7 @@ __device__ __forceinline__ void riemann_flux(const T (&L)[NV], const T (&R)[NV],
       const T ieR = (FAST && sizeof(T) == 8) ? rcp_<T, FAST>(aR - aM) : T(0);
       const T roL = divr_<T, FAST>(L[RO] * (aL - L[vn]), aL - aM, ieL);
       const T roR = divr_<T, FAST>(R[RO] * (aR - R[vn]), aR - aM, ieR);
-      // Alfven speeds; the FAST variant keeps 1/sqrt_x<T, FAST>(rho*) for the central states
+      // Alfven speeds; the FAST variant keeps 1/sqrt(rho*) for the central states
       T rsL = T(0), rsR = T(0);
       if constexpr (FAST && sizeof(T) == 8) {
         rsL = rsqrt_nr(roL);
